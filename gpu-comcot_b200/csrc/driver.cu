@@ -7,6 +7,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "fused.h"
@@ -117,11 +118,11 @@ void gc_gauge_release() {
 
 extern "C" {
 
-/* two outer steps per launch inside gcomcot_drive (kernels_pair.cu): a lone
+/* several outer steps per launch inside gcomcot_drive (kernels_block.cu): a lone
  * linear spherical outer layer with factored R2/R4, the fused path on,
  * max-eta recorded, no arrival tracking and every gauge on that layer (at
  * most 64).  GCOMCOT_DRIVE_PAIRS=0 keeps one step per launch. */
-static bool drive_pairs_ok(const GcLayer &L, int maxamp, int ngauges, const int *g_layer) {
+static bool drive_block_ok(const GcLayer &L, int maxamp, int ngauges, const int *g_layer) {
     const GcRuntime &rt = gc_rt();
     static const bool off = [] {
         const char *v = getenv("GCOMCOT_DRIVE_PAIRS");
@@ -149,10 +150,10 @@ int gcomcot_drive(int nsteps, int maxamp, int ngauges, const int *g_layer, const
     /* The caller of this entry point receives every step's stencils at the
      * end, so no step waits for the host: each step's stencils are gathered
      * on the device (by the kernel gcomcot_get_z_'s snapshot launches, at the
-     * same point of the step, or inside a two-step launch) into a history of
+     * same point of the step, or inside a launch of several steps) into a history of
      * up to kChunk steps, which goes to out4 with one copy per chunk.  Same
      * values as the per-step calls. */
-    constexpr int kChunk = 1024; /* even: a two-step launch never straddles chunks */
+    constexpr int kChunk = 1024; /* a launch never straddles chunks */
     int *d_ij = nullptr;
     float *d_hist = nullptr;
     const int chunk = nsteps < kChunk ? (nsteps > 0 ? nsteps + (nsteps & 1) : 2) : kChunk;
@@ -196,49 +197,52 @@ int gcomcot_drive(int nsteps, int maxamp, int ngauges, const int *g_layer, const
         }
     };
     int k = 0;
-    if (nsteps >= 2 && drive_pairs_ok(R, maxamp, ngauges, g_layer)) {
-        /* each launch reads the current level (buffer A) and writes the level
-         * two steps on into the other buffer (B); the intermediate level is
-         * never stored.  Its gauge stencils are recorded inside the launch.
-         * The second step's are taken by the next launch as it starts (from
-         * the level it reads), or by the gauge kernel when no launch of the
-         * same history chunk follows. */
-        constexpr int kPairVariant = 7; /* 1 warp x 5 stages, the fastest single-grid form on B200 */
+    if (nsteps >= 1 && drive_block_ok(R, maxamp, ngauges, g_layer)) {
+        /* each launch (kernels_block.cu) reads the current level (buffer A)
+         * and writes the level t steps on into the other buffer (B); the levels
+         * between are never stored.  Their gauge stencils are recorded inside
+         * the launch.  The last step's are taken by the next launch as it
+         * starts (from the level it reads), or by the gauge kernel when no
+         * launch of the same history chunk follows. */
+        int variant = 0, most = 1;
+        gc_block_form(gc_block_pick_form(1, &R.nx, &R.ny), &variant, &most);
         GcFusedGrid g;
         gc_fill_fused_grid(R, g);
+        gc_block_plan(variant, g, most);
         g.nbuf = 3;
-        g.pty = gc_pair_pick_ty(kPairVariant, 1, &R.nx, &R.ny, 2, false);
-        g.pte = gc_pair_short_ty(2, g.pty);
-        gc_pair_tiles(R.nx, R.ny, g.pty, g.pte, &g.ptiles_x);
         g.step0 = 0;
-        g.nsteps = 3; /* a launch computes local steps 0-1 or 1-2 */
+        g.nsteps = most + 2;
         g.flags = GC_F_MAXAMP | (ngauges > 0 ? GC_F_STENCIL : 0);
         g.ng = ngauges;
         g.gij = d_ij;
         g.gw = nullptr;
-        for (; k + 1 < nsteps && rc == GC_OK; k += 2) {
+        while (k < nsteps && rc == GC_OK) {
             const int A = R.cur, B = A ^ 1;
-            /* local step 1 (level buffers: read 1, write 0) when the previous
-             * step's slot is in this history chunk: the launch then also
-             * samples the level it reads into that slot; local step 0 (read
-             * 0, write 2) at a chunk's first slot */
+            /* local step 1 when the previous step's slot is in this history
+             * chunk: the launch then also samples the level it reads into that
+             * slot; local step 0 at a chunk's first slot.  Level L is in
+             * buffer L % 3, so t is not a multiple of 3. */
             const int local = (ngauges > 0 && k % chunk > 0) ? 1 : 0;
-            const int rd = local, wr = local ? 0 : 2, mid = local ? 2 : 1;
-            g.z[rd] = R.z[A]; g.m[rd] = R.m[A]; g.n[rd] = R.n[A];
-            g.z[wr] = R.z[B]; g.m[wr] = R.m[B]; g.n[wr] = R.n[B];
-            g.z[mid] = R.z[B]; g.m[mid] = R.m[B]; g.n[mid] = R.n[B];
+            int t = std::min(most, nsteps - k);
+            if (ngauges > 0) t = std::min(t, chunk - k % chunk);
+            if (t % 3 == 0) t--;
+            for (int q = 0; q < 3; q++) { /* the buffer read is level `local`'s, every other one names B */
+                g.z[q] = R.z[q == local ? A : B]; g.m[q] = R.m[q == local ? A : B];
+                g.n[q] = R.n[q == local ? A : B];
+            }
             g.ts = ngauges > 0 ? d_hist + (size_t)(k % chunk - local) * ngauges * 4 : nullptr;
             {
                 GcPdlScope pdl(true);
-                if (gc_pair_launch_one_at(kPairVariant, g, nullptr, local, rt.stream) != cudaSuccess) rc = GC_ECUDA;
+                if (gc_block_launch_one(variant, g, t, nullptr, local, rt.stream) != cudaSuccess) rc = GC_ECUDA;
             }
             rt.launches++;
+            k += t;
             if (ngauges > 0) {
-                /* the next launch samples step k + 1 when it exists and step
-                 * k + 1's slot is not the last of its chunk */
-                const bool next_samples = k + 3 < nsteps && (k + 2) % chunk != 0;
-                if (!next_samples) gauges_after(k + 1, R.z[B]);
-                flush_hist(k + 1);
+                /* the next launch samples this one's last step when it exists
+                 * and that step's slot is not the last of its chunk */
+                const bool next_samples = k < nsteps && k % chunk != 0;
+                if (!next_samples) gauges_after(k - 1, R.z[B]);
+                flush_hist(k - 1);
             }
             gc_gauge_invalidate();
             gc_swap(R);

@@ -187,6 +187,11 @@ struct gc_engine {
     bool pair_class = false;
     bool pair_class_on = true; /* GCOMCOT_PAIR_CLASS=0: always the work list */
     GcPairClass pcls;
+    /* several steps per launch, tiles in registers (kernels_block.cu) */
+    int block_on = 1;             /* the chosen candidate uses it */
+    int block_form = 0, block_variant = 0, block_T = 4;
+    int2 *d_btiles = nullptr;
+    int btiles_cap = 0, nbtiles = 0;
     int *d_health = nullptr;      /* one int for gc_engine_member_health */
     std::vector<int> nested_ids; /* active nested members */
     cudaStream_t aux[kMaxAux] = {};
@@ -376,7 +381,23 @@ static cudaError_t eng_launch_steps_(gc_engine *e, const int *d_base, int step_o
         /* two steps per launch while both lie inside every member's window
          * (the launch after a member's last step only samples its gauges) */
         int k = 0;
-        if (e->pair_ok)
+        if (e->block_on && e->pair_ok)
+            while (k < count) {
+                /* the most steps the margin, the request and the members'
+                 * windows allow; a launch must not write the buffer it reads
+                 * (level L in L % 3), and one step may also only sample */
+                int t = std::max(1, std::min({e->block_T, count - k, pair_room - k}));
+                if (t % 3 == 0) t--;
+                cudaError_t err =
+                    e->single       ? gc_block_launch_one(e->block_variant, e->one_grid, t, d_base, step_off0 + k, e->stream)
+                    : e->pair_class ? gc_block_launch_class(e->block_variant, e->pcls, t, d_base, step_off0 + k, e->stream)
+                                    : gc_block_launch_list(e->block_variant, e->d_grids, e->d_btiles, e->nbtiles, t,
+                                                           d_base, step_off0 + k, e->stream);
+                if (err != cudaSuccess) return err;
+                e->launches++;
+                k += t;
+            }
+        if (e->pair_ok && !e->block_on)
             for (; k + 1 < count && k + 2 <= pair_room; k += 2) {
                 cudaError_t err = e->single
                                       ? gc_pair_launch_one_at(e->pair_variant, e->one_grid, d_base, step_off0 + k,
@@ -441,14 +462,19 @@ static int eng_rebuild(gc_engine *e) {
         any.push_back(e->classes[M.cls].ny);
     }
     const bool single = anx.size() == 1;
+    /* until tuned: the form whose model gives these grids the shortest step */
+    if (e->block_on && !e->tuned && !anx.empty()) {
+        e->block_form = gc_block_pick_form((int)anx.size(), anx.data(), any.data());
+        gc_block_form(e->block_form, &e->block_variant, &e->block_T);
+    }
     const int ty = anx.empty() ? 16 : gc_fused_pick_ty(e->variant, (int)anx.size(), anx.data(), any.data(),
                                                        e->ty_rule, !single);
     const int pty = anx.empty() ? 32 : gc_pair_pick_ty(e->pair_variant, (int)anx.size(), anx.data(), any.data(),
                                                        e->pair_rule, !single);
     const int pte = gc_pair_short_ty(e->pair_rule, pty);
     /* two-step launches need at most 64 gauges per member */
-    bool pair_ok = e->pair_on != 0 && e->pair_allowed != 0 && !anx.empty();
-    std::vector<int2> ptiles;
+    bool pair_ok = (e->pair_on != 0 || e->block_on != 0) && e->pair_allowed != 0 && !anx.empty();
+    std::vector<int2> ptiles, btiles;
     /* active members grouped by class */
     for (size_t c = 0; c < e->classes.size(); c++) {
         EngClass &C = e->classes[c];
@@ -468,6 +494,7 @@ static int eng_rebuild(gc_engine *e) {
             g.nbuf = 3;
             g.pty = pty;
             g.pte = pte;
+            if (e->block_on) gc_block_plan(e->block_variant, g, e->block_T);
             gc_pair_tiles(C.nx, C.ny, pty, pte, &g.ptiles_x);
             for (int q = 0; q < 3; q++) { g.z[q] = M.z[q]; g.m[q] = M.m[q]; g.n[q] = M.n[q]; }
             g.h = M.h ? M.h : C.d_h; g.rows = C.d_rows;
@@ -479,9 +506,14 @@ static int eng_rebuild(gc_engine *e) {
         int nt = gc_fused_tiles(C.nx, C.ny, ty, nullptr);
         for (int t = 0; t < nt; t++)
             for (int g : idx) tiles.push_back(make_int2(g, t));
-        const int npt = gc_pair_tiles(C.nx, C.ny, pty, pte, nullptr);
+        const int npt = e->block_on ? 0 : gc_pair_tiles(C.nx, C.ny, pty, pte, nullptr);
         for (int t = 0; t < npt; t++)
             for (int g : idx) ptiles.push_back(make_int2(g, t));
+        if (e->block_on) {
+            const int nbt = grids[idx[0]].bntx * grids[idx[0]].bnty;
+            for (int t = 0; t < nbt; t++)
+                for (int g : idx) btiles.push_back(make_int2(g, t));
+        }
         for (int g : idx)
             if (grids[g].ng > 64) pair_ok = false;
     }
@@ -520,6 +552,15 @@ static int eng_rebuild(gc_engine *e) {
     if (e->nptiles)
         GC_CUDA_OR_RET(cudaMemcpyAsync(e->d_ptiles, ptiles.data(), ptiles.size() * sizeof(int2),
                                        cudaMemcpyHostToDevice, e->stream));
+    e->nbtiles = (int)btiles.size();
+    if (e->nbtiles > e->btiles_cap) {
+        if (e->d_btiles) cudaFreeAsync(e->d_btiles, e->stream);
+        e->btiles_cap = std::max(e->nbtiles, 2 * e->btiles_cap);
+        GC_CUDA_OR_RET(cudaMallocAsync((void **)&e->d_btiles, (size_t)e->btiles_cap * sizeof(int2), e->stream));
+    }
+    if (e->nbtiles)
+        GC_CUDA_OR_RET(cudaMemcpyAsync(e->d_btiles, btiles.data(), btiles.size() * sizeof(int2),
+                                       cudaMemcpyHostToDevice, e->stream));
     e->pair_ok = pair_ok;
     /* one class of single-grid members: the class launch */
     e->pair_class = false;
@@ -542,6 +583,7 @@ static int eng_rebuild(gc_engine *e) {
                 q.step0 = G.step0; q.nsteps = G.nsteps; q.flags = G.flags; q.ng = G.ng; q.ts_len = G.ts_len;
                 q.thr = G.thr;
             }
+            gc_block_class_plan(e->pcls);
             e->pair_class = true;
         }
     }
@@ -598,7 +640,11 @@ static int eng_issue(gc_engine *e, int nsteps) {
             }
         if (horizon <= 0) horizon = 1;
         if (room < 0) room = 0;
-        if (e->use_graphs && horizon >= e->chunk && (!e->pair_ok || room >= e->chunk)) {
+        /* the register-tile launches last longer than the host takes to issue
+         * one, so without nested chains they go out as they are, and no graph
+         * has to be captured when the members change */
+        const bool graphs = e->use_graphs && !(e->block_on && e->pair_ok && e->nested_ids.empty());
+        if (graphs && horizon >= e->chunk && (!e->pair_ok || room >= e->chunk)) {
             /* the device counter must equal the host's step count */
             GC_CUDA_OR_RET(cudaMemcpyAsync(e->d_step, &e->gstep, sizeof(int), cudaMemcpyHostToDevice, e->stream));
             if (!e->gexec) GC_CUDA_OR_RET(eng_build_graph(e));
@@ -645,11 +691,11 @@ int gc_engine_create(long long hbm_budget_bytes, gc_engine **out) {
         return GC_ECUDA;
     }
     const char *v = getenv("GCOMCOT_FUSED_VARIANT");
-    if (v) { e->variant = atoi(v); e->tuned = true; }
+    if (v) { e->variant = atoi(v); e->tuned = true; e->block_on = 0; }
     const char *pd = getenv("GCOMCOT_PDL");
     if (pd && pd[0] == '0') e->pdl = 0;
     const char *pr = getenv("GCOMCOT_PAIR");
-    if (pr && pr[0] == '0') e->pair_on = e->pair_allowed = 0;
+    if (pr && pr[0] == '0') e->pair_on = e->pair_allowed = e->block_on = 0;
     const char *pc = getenv("GCOMCOT_PAIR_CLASS");
     if (pc && pc[0] == '0') e->pair_class_on = false;
     *out = e;
@@ -670,6 +716,7 @@ int gc_engine_destroy(gc_engine *e) {
     if (e->d_grids) cudaFreeAsync(e->d_grids, e->stream);
     if (e->d_tiles) cudaFreeAsync(e->d_tiles, e->stream);
     if (e->d_ptiles) cudaFreeAsync(e->d_ptiles, e->stream);
+    if (e->d_btiles) cudaFreeAsync(e->d_btiles, e->stream);
     if (e->d_step) cudaFreeAsync(e->d_step, e->stream);
     if (e->d_health) cudaFreeAsync(e->d_health, e->stream);
     cudaStreamSynchronize(e->stream);
@@ -1169,14 +1216,21 @@ long long gc_engine_bytes_in_use(gc_engine *e) { return e ? e->in_use : GC_EINVA
  * tile-height rule c / nv; above that the two-step kernel, variant p % np
  * with rule p / np (p = c - nv * R1) */
 
+/* the register-tile kernel's forms follow */
 static int eng_num_candidates() {
-    return gc_fused_num_variants() * GC_TY_RULES + gc_pair_num_variants() * GC_PAIR_RULES;
+    return gc_fused_num_variants() * GC_TY_RULES + gc_pair_num_variants() * GC_PAIR_RULES + gc_block_num_forms();
 }
 
 static bool eng_set_candidate(gc_engine *e, int c) {
     const int nv = gc_fused_num_variants(), n1 = nv * GC_TY_RULES, np = gc_pair_num_variants();
     if (c < 0 || c >= eng_num_candidates()) return false;
-    if (c < n1) {
+    const int n2 = n1 + np * GC_PAIR_RULES;
+    e->block_on = 0;
+    if (c >= n2) {
+        e->block_form = c - n2;
+        gc_block_form(e->block_form, &e->block_variant, &e->block_T);
+        e->block_on = 1;
+    } else if (c < n1) {
         e->variant = c % nv;
         e->ty_rule = c / nv;
         e->pair_on = 0;
@@ -1224,8 +1278,9 @@ int gc_engine_autotune(gc_engine *e, int reps) {
     auto time_candidate = [&](int c, int rounds, int chunks = 0) -> float {
         eng_set_candidate(e, c);
         e->use_graphs = chunks > 0 ? saved_graphs : 0;
-        const int n = chunks > 0 ? chunks * e->chunk : (c >= n1 ? 2 * reps : reps) * rounds;
-        if (eng_issue(e, chunks > 0 ? e->chunk : (c >= n1 ? 2 : 1)) < 0) return -1.0f; /* warm */
+        const int per = e->block_on ? e->block_T : c >= n1 ? 2 : 1; /* steps per launch */
+        const int n = chunks > 0 ? chunks * e->chunk : per * reps * rounds;
+        if (eng_issue(e, chunks > 0 ? e->chunk : per) < 0) return -1.0f; /* warm */
         cudaEventRecord(a, e->stream);
         int got = eng_issue(e, n);
         cudaEventRecord(b, e->stream);
@@ -1276,7 +1331,8 @@ int gc_engine_prepare(gc_engine *e) {
     if (!e) return GC_EINVAL;
     eng_retire(e);
     if (e->dirty && eng_rebuild(e) != GC_OK) return GC_ECUDA;
-    if (e->use_graphs && !e->gexec && (e->ntiles > 0 || !e->nested_ids.empty()))
+    if (e->use_graphs && !e->gexec && (e->ntiles > 0 || !e->nested_ids.empty()) &&
+        !(e->block_on && e->pair_ok && e->nested_ids.empty()))
         GC_CUDA_OR_RET(eng_build_graph(e));
     GC_CUDA_OR_RET(cudaStreamSynchronize(e->stream));
     return GC_OK;
@@ -1284,6 +1340,8 @@ int gc_engine_prepare(gc_engine *e) {
 
 int gc_engine_variant(gc_engine *e) {
     if (!e) return GC_EINVAL;
+    if (e->block_on && e->pair_allowed)
+        return gc_fused_num_variants() * GC_TY_RULES + gc_pair_num_variants() * GC_PAIR_RULES + e->block_form;
     if (e->pair_on && e->pair_allowed)
         return gc_fused_num_variants() * GC_TY_RULES + e->pair_variant + gc_pair_num_variants() * e->pair_rule;
     return e->variant + gc_fused_num_variants() * e->ty_rule;

@@ -49,6 +49,11 @@ struct GcFusedGrid {
      * max-eta or arrival update, since a nested child's feedback rewrites
      * their surface after this launch (zero-filled descriptors have none) */
     int has_win, wi0, wi1, wj0, wj1;
+    /* register-tile kernel: margin rows of a window (the most steps a launch
+     * may take), windows along I and J, windows on the perimeter (numbered
+     * first), ceil(2^32 / windows of an inner row) */
+    int bt, bntx, bnty, bper;
+    unsigned bmag;
 };
 
 /* one launch variant: warps per CTA and pipeline stages per warp */
@@ -119,6 +124,7 @@ struct GcPairMember {
 struct GcPairClass {
     GcFusedGrid proto; /* the geometry; its member fields are not read */
     int nm, ntiles;    /* members, tiles per member */
+    unsigned mag;      /* register-tile kernel: ceil(2^32 / nm) */
     GcPairMember m[GC_PAIR_CLASS_MAX];
 };
 cudaError_t gc_pair_launch_class(int variant, const GcPairClass &c, const int *d_step_base, int step_off,
@@ -135,5 +141,28 @@ void gc_pair_set_wait_limit(int polls);
 /* the next two-step launch makes its first warp wait for a row nothing
  * delivers (no copy is issued for it): the bounded wait then gives up */
 void gc_pair_stall_next();
+
+/* ---- several steps per launch, tiles in registers (kernels_block.cu): the
+ * outermost layer only, factored R2/R4, arrival by max-eta, at most 64
+ * gauges.  A grid's `bt` is the most steps a launch takes; a launch of T <= bt
+ * steps reads level L and writes L + T.  With nbuf 3 level L + T must not
+ * share L's buffer (T % 3 != 0); with nbuf 2 T is 1. ---- */
+/* the forms of a launch (window shape, most steps), and the one expected to
+ * be fastest for a set of grids stepped together */
+int gc_block_num_forms();
+void gc_block_form(int form, int *variant, int *steps);
+int gc_block_pick_form(int ngrids, const int *nx, const int *ny);
+/* fills a grid's window layout for launches of up to bt steps; returns the
+ * number of windows */
+int gc_block_plan(int variant, GcFusedGrid &g, int bt);
+void gc_block_class_plan(GcPairClass &c);
+cudaError_t gc_block_launch_one(int variant, const GcFusedGrid &g, int T, const int *d_step_base, int step_off,
+                                cudaStream_t s);
+/* tiles[k] = {grid, window} */
+cudaError_t gc_block_launch_list(int variant, const GcFusedGrid *d_grids, const int2 *d_tiles,
+                                 int ntiles, int T, const int *d_step_base, int step_off, cudaStream_t s);
+/* the members of one class; proto.bt is the class's margin */
+cudaError_t gc_block_launch_class(int variant, const GcPairClass &c, int T, const int *d_step_base, int step_off,
+                                  cudaStream_t s);
 
 #endif
