@@ -209,6 +209,7 @@ int gcomcot_drive(int nsteps, int maxamp, int ngauges, const int *g_layer, const
         GcFusedGrid g;
         gc_fill_fused_grid(R, g);
         gc_block_plan(variant, g, most);
+        const bool fits = gc_block_fits(g, 1); /* else one step at a time below */
         g.nbuf = 3;
         g.step0 = 0;
         g.nsteps = most + 2;
@@ -216,7 +217,7 @@ int gcomcot_drive(int nsteps, int maxamp, int ngauges, const int *g_layer, const
         g.ng = ngauges;
         g.gij = d_ij;
         g.gw = nullptr;
-        while (k < nsteps && rc == GC_OK) {
+        while (fits && k < nsteps && rc == GC_OK) {
             const int A = R.cur, B = A ^ 1;
             /* local step 1 when the previous step's slot is in this history
              * chunk: the launch then also samples the level it reads into that

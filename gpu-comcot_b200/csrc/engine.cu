@@ -85,7 +85,6 @@ struct EngMember {
      * step has written the outer grid's real level 2 by then) */
     float *sm2 = nullptr, *sn2 = nullptr;
     float *h = nullptr; /* own depth (members made from faults), else the class's */
-    int fty = 16; /* tile height of the outer grid's fused launch */
     /* the last global step this member needs a launch at: single-grid
      * members sample their last gauges in the launch after their last step */
     int last_step() const { return nested ? step0 + nsteps - 1 : step0 + nsteps; }
@@ -234,9 +233,7 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
     GcFusedGrid g;
     memset(&g, 0, sizeof g);
     g.nx = C.nx; g.ny = C.ny; g.pitch = C.pitch; g.root = 1; g.explicit_r24 = 0;
-    g.ty = M.fty;
-    gc_fused_tiles(C.nx, C.ny, g.ty, &g.tiles_x);
-    /* the fused launch records max-eta and arrival outside the JNZ window
+    /* the step's launch records max-eta and arrival outside the JNZ window
      * (IS..IE x JS..JE, 0-based IS-1..IE-1); the outputs kernel does the window */
     const int win[4] = {C.corners[0] - 1, C.corners[1] - 1, C.corners[2] - 1, C.corners[3] - 1};
     const int flags = GC_F_MAXAMP | (M.thr >= 0.0f ? GC_F_ARRIVAL | GC_F_ARR_BYMAX : 0);
@@ -287,7 +284,7 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
         e->launches += pre + gc_launch_moment_update(Cv1, cs);
     }
     cudaEventRecord(e->ev_cjoin[a], cs);
-    gc_fused_launch_one_at(e->variant, g, d_base, step_off, s);
+    gc_step_launch_one(g, d_base, step_off, s);
     cudaStreamWaitEvent(s, e->ev_cjoin[a], 0);
     auto jnz = [&](const GcLayerDev &Cv) {
         if (C.has_sc) gc_launch_sc_jnz(P, Cv, C.sc, s);
@@ -475,6 +472,7 @@ static int eng_rebuild(gc_engine *e) {
     /* two-step launches need at most 64 gauges per member */
     bool pair_ok = (e->pair_on != 0 || e->block_on != 0) && e->pair_allowed != 0 && !anx.empty();
     std::vector<int2> ptiles, btiles;
+    bool block_fits = true; /* fields beyond 4 GB go through the one-step kernel */
     /* active members grouped by class */
     for (size_t c = 0; c < e->classes.size(); c++) {
         EngClass &C = e->classes[c];
@@ -509,7 +507,8 @@ static int eng_rebuild(gc_engine *e) {
         const int npt = e->block_on ? 0 : gc_pair_tiles(C.nx, C.ny, pty, pte, nullptr);
         for (int t = 0; t < npt; t++)
             for (int g : idx) ptiles.push_back(make_int2(g, t));
-        if (e->block_on) {
+        if (e->block_on && !gc_block_fits(grids[idx[0]], (int)idx.size())) block_fits = false;
+        if (e->block_on && block_fits) {
             const int nbt = grids[idx[0]].bntx * grids[idx[0]].bnty;
             for (int t = 0; t < nbt; t++)
                 for (int g : idx) btiles.push_back(make_int2(g, t));
@@ -518,11 +517,6 @@ static int eng_rebuild(gc_engine *e) {
             if (grids[g].ng > 64) pair_ok = false;
     }
     if (eng_make_aux(e, (int)e->nested_ids.size()) != GC_OK) return GC_ECUDA;
-    /* the outer grid of a nested member is stepped alone on its own stream */
-    for (int id : e->nested_ids) {
-        EngMember &M = e->members[id];
-        M.fty = gc_fused_pick_ty(e->variant, 1, &e->classes[M.cls].nx, &e->classes[M.cls].ny, 1, false);
-    }
     e->ngrids = (int)grids.size();
     e->ntiles = (int)tiles.size();
     e->single = single && e->ngrids == 1;
@@ -552,6 +546,7 @@ static int eng_rebuild(gc_engine *e) {
     if (e->nptiles)
         GC_CUDA_OR_RET(cudaMemcpyAsync(e->d_ptiles, ptiles.data(), ptiles.size() * sizeof(int2),
                                        cudaMemcpyHostToDevice, e->stream));
+    if (!block_fits) pair_ok = false;
     e->nbtiles = (int)btiles.size();
     if (e->nbtiles > e->btiles_cap) {
         if (e->d_btiles) cudaFreeAsync(e->d_btiles, e->stream);

@@ -78,8 +78,8 @@ cudaError_t gc_fused_launch_multi(int variant, const GcFusedGrid *d_grids, const
 int gc_fused_max_ctas(int variant, bool multi = true);
 /* 1 if a pipeline wait in the fused kernel gave up since the last call (clears it) */
 int gc_fused_take_error();
-/* clears that flag in stream order on `s` */
-cudaError_t gc_fused_clear_error_async(cudaStream_t s);
+/* that flag's device address */
+cudaError_t gc_fused_error_flag(int **flag);
 /* single grid, descriptor by value */
 cudaError_t gc_fused_launch_one(int variant, const GcFusedGrid &g, int step, cudaStream_t s);
 /* single grid at step step_off + *d_step_base (d_step_base may be NULL) */
@@ -152,6 +152,9 @@ void gc_pair_stall_next();
 int gc_block_num_forms();
 void gc_block_form(int form, int *variant, int *steps);
 int gc_block_pick_form(int ngrids, const int *nx, const int *ny);
+/* whether a planned grid's byte offsets and window numbers fit 32 bits
+ * (`members` of them in a class launch) */
+bool gc_block_fits(const GcFusedGrid &g, int members);
 /* fills a grid's window layout for launches of up to bt steps; returns the
  * number of windows */
 int gc_block_plan(int variant, GcFusedGrid &g, int bt);
@@ -164,5 +167,11 @@ cudaError_t gc_block_launch_list(int variant, const GcFusedGrid *d_grids, const 
 /* the members of one class; proto.bt is the class's margin */
 cudaError_t gc_block_launch_class(int variant, const GcPairClass &c, int T, const int *d_step_base, int step_off,
                                   cudaStream_t s);
+
+/* ---- one step, warps on their own (kernels_step.cu): factored R2/R4, the
+ * outermost layer, no gauges, arrival by max-eta ---- */
+cudaError_t gc_step_launch_one(const GcFusedGrid &g, const int *d_step_base, int step_off, cudaStream_t s);
+/* up to 64 grids by value; clear: a device flag to set to 0, or NULL */
+cudaError_t gc_step_launch_grids(int n, const GcFusedGrid *g, int step, int *clear, cudaStream_t s);
 
 #endif

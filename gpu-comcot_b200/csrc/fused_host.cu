@@ -36,21 +36,27 @@ bool gc_fused_step(GcLayer &L, bool maxamp, bool arrival, int step, float thr, i
     if (L.parent != -1 && !L.children.empty()) return false;
     GcFusedGrid g;
     gc_fill_fused_grid(L, g);
-    int v = gc_default_variant();
-    static int cached_nx = -1, cached_ny = -1, cached_v = -1, cached_ty = 16;
-    if (cached_nx != L.nx || cached_ny != L.ny || cached_v != v) {
-        /* the single-grid kernel; rule 1 (fewest rows for the busiest warp) */
-        cached_ty = gc_fused_pick_ty(v, 1, &L.nx, &L.ny, 1, false);
-        cached_nx = L.nx; cached_ny = L.ny; cached_v = v;
-    }
-    g.ty = cached_ty;
-    gc_fused_tiles(L.nx, L.ny, g.ty, &g.tiles_x);
     g.step0 = step;
     g.cur0 = L.cur;
     g.nsteps = 0x3fffffff;
     g.flags = (maxamp ? GC_F_MAXAMP : 0) | (arrival ? GC_F_ARRIVAL : 0);
     g.thr = thr;
-    cudaError_t e = gc_fused_launch_one(v, g, step, s);
+    cudaError_t e;
+    if (!g.explicit_r24 && !arrival) {
+        e = gc_step_launch_one(g, nullptr, step, s);
+    } else {
+        /* R2 and R4 as fields: the kernel that streams them */
+        int v = gc_default_variant();
+        static int cached_nx = -1, cached_ny = -1, cached_v = -1, cached_ty = 16;
+        if (cached_nx != L.nx || cached_ny != L.ny || cached_v != v) {
+            /* the single-grid kernel; rule 1 (fewest rows for the busiest warp) */
+            cached_ty = gc_fused_pick_ty(v, 1, &L.nx, &L.ny, 1, false);
+            cached_nx = L.nx; cached_ny = L.ny; cached_v = v;
+        }
+        g.ty = cached_ty;
+        gc_fused_tiles(L.nx, L.ny, g.ty, &g.tiles_x);
+        e = gc_fused_launch_one(v, g, step, s);
+    }
     if (e != cudaSuccess) {
         fprintf(stderr, "gcomcot: fused launch failed: %s\n", cudaGetErrorString(e));
         exit(EXIT_FAILURE);

@@ -668,13 +668,7 @@ int gc_fused_take_error() {
     return v;
 }
 
-/* clears the pipeline-error flag in stream order (no host memory involved) */
-cudaError_t gc_fused_clear_error_async(cudaStream_t s) {
-    void *addr = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&addr, g_pipe_error);
-    if (e != cudaSuccess) return e;
-    return cudaMemsetAsync(addr, 0, sizeof(int), s);
-}
+cudaError_t gc_fused_error_flag(int **flag) { return cudaGetSymbolAddress((void **)flag, g_pipe_error); }
 
 GcTileCfg gc_fused_variant(int v) {
     if (v < 0 || v >= kNumVariants) v = 0;

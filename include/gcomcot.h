@@ -290,15 +290,12 @@ typedef struct {
  * memory (codes that own all device memory, pipelines with a fixed reserved
  * budget, loops where an allocation's device synchronisation is not
  * acceptable): one outer step (MASS_S + OPEN + MOMT_S + max) of every grid in
- * one launch on `stream`, with its work list in a fixed array built into the
- * library (at most 64 grids and 24576 tiles of 128 columns; larger requests
- * return -1).  The grid list travels in the launch parameters of a small
- * kernel that fills the array, so nothing is copied from host memory and the
- * call returns once its work is queued.  Calls share that array: calls that
- * overlap on the GPU race.  The first call on a device does a one-time set-up
- * and should come before any stream capture.  A bounded pipeline wait that
- * gives up is reported by gcomcot_sync() (GC_ETIMEOUT) after the caller has
- * synchronised `stream`.  Returns 0 or a negative status. */
+ * one launch on `stream` (at most 64 grids, and 24576 tiles of 128 columns by
+ * 4096 rows; larger requests return -1).  The grid list travels in the launch
+ * parameters, so nothing is copied from host memory, the library holds no
+ * device memory for it, and the call returns once its launch is queued.  The
+ * first call on a device does a one-time set-up and should come before any
+ * stream capture.  Returns 0 or a negative status. */
 int gcomcot_fused_step_noalloc(int ngrids, const gc_grid_step_io *grids, void *stream);
 
 #ifdef __cplusplus
