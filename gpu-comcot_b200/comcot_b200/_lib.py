@@ -99,6 +99,7 @@ SIGNATURES = {
     "gc_event_release": (C.c_int, [VP]),
     "gc_host_alloc": (VP, [C.c_longlong]),
     "gc_host_free": (C.c_int, [VP]),
+    "gc_host_copy": (C.c_int, [VP, VP, C.c_longlong]),
     "gc_engine_bytes_in_use": (C.c_longlong, [VP]),
     "gc_engine_member_bytes": (C.c_longlong, [VP, C.c_int]),
     "gc_engine_config": (C.c_int, [VP, C.c_int, C.c_int, C.c_int]),

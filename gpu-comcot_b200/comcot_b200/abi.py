@@ -173,26 +173,26 @@ class ReferenceSession:
 
     def getz(self, lid=1):
         L = self._layer(lid)
-        z = np.zeros((L.ny, L.nx), F32)
+        z = np.empty((L.ny, L.nx), F32)
         self.lib.cuda_getz_(_lib.fptr(z), _i(lid))
         return z
 
     def getmn(self, lid=1):
         L = self._layer(lid)
-        m = np.zeros((L.ny, L.nx), F32)
-        n = np.zeros((L.ny, L.nx), F32)
+        m = np.empty((L.ny, L.nx), F32)
+        n = np.empty((L.ny, L.nx), F32)
         self.lib.cuda_getmn_(_lib.fptr(m), _lib.fptr(n), _i(lid))
         return m, n
 
     def getzmax(self, lid=1):
         L = self._layer(lid)
-        z = np.zeros((L.ny, L.nx), F32)
+        z = np.empty((L.ny, L.nx), F32)
         self.lib.cuda_getzmax_(_lib.fptr(z), _i(lid))
         return z
 
     def getarrival(self, lid=1):
         L = self._layer(lid)
-        a = np.zeros((L.ny, L.nx), np.int32)
+        a = np.empty((L.ny, L.nx), np.int32)
         self.lib.gcomcot_get_arrival_(_lib.iptr(a), _i(lid))
         return a
 

@@ -59,7 +59,11 @@ class PendingRead:
         rc = self.lib.gc_event_wait(self.event)
         if rc != 0:
             raise RuntimeError(f"gc_event_wait failed: {rc}")
-        out = {k: np.array(v, copy=True) for k, v in self.views.items()}
+        out = {}
+        for k, v in self.views.items():
+            out[k] = np.empty(v.shape, v.dtype)
+            if v.nbytes:
+                self.lib.gc_host_copy(out[k].ctypes.data, v.ctypes.data, v.nbytes)
         self.lib.gc_event_release(self.event)
         self.pool.give(self.nbytes, self.ptr)
         self.event = None
@@ -249,9 +253,9 @@ class Engine:
         out = {}
         for k in ("z", "m", "n", "zmax"):
             if k in want:
-                out[k] = np.zeros((ny, nx), F32)
+                out[k] = np.empty((ny, nx), F32)
         if "arrival" in want:
-            out["arrival"] = np.zeros((ny, nx), np.int32)
+            out["arrival"] = np.empty((ny, nx), np.int32)
         if "ts" in want:
             out["ts"] = np.zeros((n, max(ng, 1)), F32)
         rc = self.lib.gc_engine_read(self.h, mid, _lib.fptr(out.get("z")), _lib.fptr(out.get("m")),
@@ -265,7 +269,7 @@ class Engine:
         if child is not None and ("child" in want or "z" in want):
             cnx, cny = child
             for k in ("child_z", "child_m", "child_n"):
-                out[k] = np.zeros((cny, cnx), F32)
+                out[k] = np.empty((cny, cnx), F32)
             rc = self.lib.gc_engine_read_child(self.h, mid, _lib.fptr(out["child_z"]), _lib.fptr(out["child_m"]),
                                                _lib.fptr(out["child_n"]))
             if rc != 0:

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "fused.h"
+#include "hostio.h"
 #include "runtime.h"
 
 bool gc_fused_step(GcLayer &L, bool maxamp, bool arrival, int step, float thr, int ngauges,
@@ -83,10 +84,8 @@ void gcomcot_get_arrival_(int *arr, int *id) {
     GcLayer *L = gc_layer(*id);
     if (!L || !L->used) exit(EXIT_FAILURE);
     gc_flush();
-    GC_CUDA_OR_DIE(cudaMemcpy2DAsync(arr, (size_t)L->nx * sizeof(int), L->arrival,
-                                     (size_t)L->pitch * sizeof(int), (size_t)L->nx * sizeof(int),
-                                     (size_t)L->ny, cudaMemcpyDeviceToHost, gc_rt().stream));
-    GC_CUDA_OR_DIE(cudaStreamSynchronize(gc_rt().stream));
+    if (gc_field_download(arr, L->arrival, (size_t)L->pitch * sizeof(int), L->nx, L->ny, gc_rt().stream) != GC_OK)
+        exit(EXIT_FAILURE);
 }
 
 /* number of kernels this library has launched since initialisation */

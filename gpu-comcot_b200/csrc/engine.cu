@@ -37,6 +37,7 @@
 
 #include "fused.h"
 #include "gcomcot.h"
+#include "hostio.h"
 
 namespace {
 
@@ -824,9 +825,8 @@ static int eng_add_member(gc_engine *e, int cls, const float *z0, const float *c
             return rc;
         }
     } else {
-        GC_CUDA_OR_RET(cudaMemcpy2DAsync(M.z[0], (size_t)C.pitch * sizeof(float), z0, (size_t)C.nx * sizeof(float),
-                                         (size_t)C.nx * sizeof(float), (size_t)C.ny, cudaMemcpyHostToDevice,
-                                         e->stream));
+        int rc = gc_field_upload(M.z[0], (size_t)C.pitch * sizeof(float), z0, C.nx, C.ny, e->stream);
+        if (rc != GC_OK) return rc;
     }
     GC_CUDA_OR_RET(cudaMemcpyAsync(M.zmax, M.z[0], field, cudaMemcpyDeviceToDevice, e->stream));
     if (arrival_thr >= 0.0f) {
@@ -1073,15 +1073,15 @@ int gc_engine_read(gc_engine *e, int id, float *z, float *m, float *n, float *zm
     /* level 1 after the member's completed steps */
     int done_steps = std::min(std::max(e->gstep - M.step0 + 1, 0), M.nsteps);
     int cur = M.level_buf(done_steps);
-    size_t sp = (size_t)C.pitch * sizeof(float), dp = (size_t)C.nx * sizeof(float);
     auto dl = [&](void *dst, const void *src) {
-        return cudaMemcpy2DAsync(dst, dp, src, sp, dp, (size_t)C.ny, cudaMemcpyDeviceToHost, e->stream);
+        return dst ? gc_field_download(dst, src, (size_t)C.pitch * sizeof(float), C.nx, C.ny, e->stream) : GC_OK;
     };
-    if (z) GC_CUDA_OR_RET(dl(z, M.z[cur]));
-    if (m) GC_CUDA_OR_RET(dl(m, M.m[cur]));
-    if (n) GC_CUDA_OR_RET(dl(n, M.n[cur]));
-    if (zmax) GC_CUDA_OR_RET(dl(zmax, M.zmax));
-    if (arrival) GC_CUDA_OR_RET(dl(arrival, M.arrival));
+    int rc = dl(z, M.z[cur]);
+    if (rc == GC_OK) rc = dl(m, M.m[cur]);
+    if (rc == GC_OK) rc = dl(n, M.n[cur]);
+    if (rc == GC_OK) rc = dl(zmax, M.zmax);
+    if (rc == GC_OK) rc = dl(arrival, M.arrival);
+    if (rc != GC_OK) return rc;
     if (ts && M.ng > 0)
         GC_CUDA_OR_RET(cudaMemcpyAsync(ts, M.ts, (size_t)M.nsteps * M.ng * sizeof(float), cudaMemcpyDeviceToHost,
                                        e->stream));
@@ -1154,13 +1154,13 @@ int gc_engine_read_child(gc_engine *e, int id, float *z, float *m, float *n) {
     EngClass &C = e->classes[M.cls];
     int done_steps = std::min(std::max(e->gstep - M.step0 + 1, 0), M.nsteps);
     int cur = (int)(((long long)done_steps * C.rel_time) & 1);
-    size_t sp = (size_t)C.cpitch * sizeof(float), dp = (size_t)C.cnx * sizeof(float);
     auto dl = [&](void *dst, const void *src) {
-        return cudaMemcpy2DAsync(dst, dp, src, sp, dp, (size_t)C.cny, cudaMemcpyDeviceToHost, e->stream);
+        return dst ? gc_field_download(dst, src, (size_t)C.cpitch * sizeof(float), C.cnx, C.cny, e->stream) : GC_OK;
     };
-    if (z) GC_CUDA_OR_RET(dl(z, M.cz[cur]));
-    if (m) GC_CUDA_OR_RET(dl(m, M.cm[cur]));
-    if (n) GC_CUDA_OR_RET(dl(n, M.cn[cur]));
+    int rc = dl(z, M.cz[cur]);
+    if (rc == GC_OK) rc = dl(m, M.cm[cur]);
+    if (rc == GC_OK) rc = dl(n, M.cn[cur]);
+    if (rc != GC_OK) return rc;
     GC_CUDA_OR_RET(cudaStreamSynchronize(e->stream));
     return GC_OK;
 }

@@ -23,6 +23,7 @@
 #include <thread>
 #include <vector>
 
+#include "hostio.h"
 #include "runtime.h"
 
 void gc_gauge_invalidate();
@@ -135,19 +136,12 @@ int gc_layer_alloc(GcLayer &L) {
 }
 
 int gc_layer_upload_field(GcLayer &L, float *dst, const float *src) {
-    GC_CUDA_OR_RET(cudaMemcpy2DAsync(dst, (size_t)L.pitch * sizeof(float), src,
-                                     (size_t)L.nx * sizeof(float), (size_t)L.nx * sizeof(float),
-                                     (size_t)L.ny, cudaMemcpyHostToDevice, g_rt.stream));
-    GC_CUDA_OR_RET(cudaStreamSynchronize(g_rt.stream));
-    return GC_OK;
+    /* the caller's array has been read when this returns */
+    return gc_field_upload(dst, (size_t)L.pitch * sizeof(float), src, L.nx, L.ny, g_rt.stream);
 }
 
 int gc_layer_download_field(GcLayer &L, const float *src, float *dst) {
-    GC_CUDA_OR_RET(cudaMemcpy2DAsync(dst, (size_t)L.nx * sizeof(float), src,
-                                     (size_t)L.pitch * sizeof(float), (size_t)L.nx * sizeof(float),
-                                     (size_t)L.ny, cudaMemcpyDeviceToHost, g_rt.stream));
-    GC_CUDA_OR_RET(cudaStreamSynchronize(g_rt.stream));
-    return GC_OK;
+    return gc_field_download(dst, src, (size_t)L.pitch * sizeof(float), L.nx, L.ny, g_rt.stream);
 }
 
 /* R2 = C(J) * AMAX1(HP(I,J),0) (comcot.f90:733-736) with HP from PQ_DEPTH

@@ -196,6 +196,9 @@ int gc_event_release(void *event);
 /* page-locked host memory for asynchronous reads (NULL when refused) */
 void *gc_host_alloc(long long bytes);
 int gc_host_free(void *p);
+/* copies between host blocks that do not overlap, by several threads where
+ * that is faster (results out of page-locked blocks into ordinary arrays) */
+int gc_host_copy(void *dst, const void *src, long long bytes);
 
 /* A nested grid class: the outer grid of class `parent_cls` with one child
  * layer (ALL_GRID sub-cycle, all_grids.f90:4-312).
