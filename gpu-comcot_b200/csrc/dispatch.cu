@@ -40,6 +40,10 @@ void gc_flush() {
         done = gc_fused_step(L, rt.pend_maxamp != 0, false, 0, 0.0f, 0, nullptr, nullptr, rt.stream);
         if (done) rt.launches++;
     }
+    if (!done && rt.fuse_enabled && rt.pend_mass && rt.pend_open && rt.pend_momt) {
+        done = gc_launch_root_step(L.view(), rt.pend_maxamp != 0, rt.stream);
+        if (done) rt.launches++;
+    }
     if (!done) {
         GcLayerDev d = L.view();
         if (rt.pend_mass) { gc_launch_mass(d, rt.stream); rt.launches++; }

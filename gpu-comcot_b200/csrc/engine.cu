@@ -262,12 +262,16 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
     if (C.has_sc) { Pf.m2 = M.sm2; Pf.n2 = M.sn2; }
     cudaEventRecord(e->ev_cfork[a], s);
     cudaStreamWaitEvent(cs, e->ev_cfork[a], 0);
-    /* edge fluxes and mass: one launch for a Cartesian child (JNQ's values
-     * computed where the mass reads them), two otherwise */
+    /* a nonlinear child's sub-step is one launch; else edge fluxes and mass
+     * are one for a Cartesian child (JNQ's values computed where the mass
+     * reads them), two otherwise */
     int pre = 2;
+    bool whole = false;
     if (C.has_sc) {
         gc_launch_sc_edges(Pf, Cv1, C.sc, 1, C.rel_time, Cv1.z1, cs);
         gc_launch_mass(Cv1, cs);
+    } else if (gc_launch_child_step(P, Cv1, C.rel_size, C.rel_time, C.corners, 1, cs)) {
+        whole = true;
     } else if (gc_launch_edges_mass(P, Cv1, C.rel_size, C.rel_time, C.corners, 1, cs)) {
         pre = 1;
     } else {
@@ -278,7 +282,9 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
      * 0 included, so in the sub-step that feeds back UPDATE's edge copy
      * follows it (all_grids.f90 order: MOMENT, JNZ, UPDATE) */
     const bool late_update1 = C.has_sc && nhalf == 1;
-    if (late_update1) {
+    if (whole) {
+        e->launches++;
+    } else if (late_update1) {
         gc_launch_moment(Cv1, cs);
         e->launches += pre + 1;
     } else {
@@ -303,6 +309,12 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
     cc ^= 1;
     for (int t = 2; t <= C.rel_time; t++) {
         const GcLayerDev Cv = child_view(C, M, cc);
+        if (!C.has_sc && gc_launch_child_step(P, Cv, C.rel_size, C.rel_time, C.corners, t, s)) {
+            e->launches++;
+            if (t == nhalf) jnz(Cv);
+            cc ^= 1;
+            continue;
+        }
         if (C.has_sc) {
             gc_launch_sc_forecast(Pf, C.sc, s);
             gc_launch_sc_edges(Pf, Cv, C.sc, t, C.rel_time, Cv.z1, s);

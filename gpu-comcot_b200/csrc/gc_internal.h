@@ -115,6 +115,14 @@ void gc_launch_jnz(const GcLayerDev &P, const GcLayerDev &C, int rel_size, int r
  * other child kinds): then call gc_launch_edges and gc_launch_mass */
 bool gc_launch_edges_mass(const GcLayerDev &P, const GcLayerDev &C, int rel_size, int rel_time,
                           const int *corners, int t, cudaStream_t s);
+/* sub-step t of a nonlinear child without children of its own and without
+ * SC_OPTION = 1: edge fluxes, mass, momentum and UPDATE's edge copy in one
+ * launch; false (nothing launched) for other children */
+bool gc_launch_child_step(const GcLayerDev &P, const GcLayerDev &C, int rel_size, int rel_time, const int *corners,
+                          int t, cudaStream_t s);
+/* a nonlinear root layer's mass, OPEN, momentum and, maxamp, maximum in one
+ * launch; false (nothing launched) for other layers */
+bool gc_launch_root_step(const GcLayerDev &L, bool maxamp, cudaStream_t s);
 /* SC_OPTION = 1 coupling of a Cartesian child to a spherical parent: the
  * parent cell (KI, KJ) and bilinear weights of every child edge node, and
  * for JNZ_SC, per parent cell of the child's window, the child nodes that

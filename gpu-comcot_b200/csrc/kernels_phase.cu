@@ -437,20 +437,24 @@ __device__ __forceinline__ float face2(float a, float b) {
     return v < CC_GX ? 0.0f : v;
 }
 
-/* WAVE_BREAKING (moment.f90:1302-1335) on one cell's total depth, new and
- * old surface */
-__device__ __forceinline__ void wave_breaking(float dz2c, float z2c, float z1c, float dt, float &advx,
-                                              float &advy) {
+/* WAVE_BREAKING (moment.f90:1302-1335) on one cell's total depth, new and old
+ * surface: the damping coefficient of the advection terms of both the cell's
+ * faces, < 0 where the wave does not break.  It breaks where |dZ|/dt exceeds
+ * 0.08 sqrt(g d); where the squares are apart by more than 1.5 % (0.0063 for
+ * 0.08^2), far beyond any rounding, the square root and the division are not
+ * needed to know that it does not. */
+__device__ __forceinline__ float breaking(float dz2c, float z2c, float z1c, float dt) {
+    const float a = fabs_(z2c - z1c);
+    if (a * a < 0.0063f * (dt * dt) * (CC_GRAV * dz2c)) return -1.0f;
     float cc = sqrtf(CC_GRAV * dz2c);
     float dzdt_f = CC_BRK_F * cc;
     float dzdt_i = CC_BRK_I * cc;
-    float dzdt = qdiv(fabs_(z2c - z1c), dt);
+    float dzdt = qdiv(a, dt);
     if (dzdt > dzdt_f) {
         float ref = (dzdt - dzdt_f) / (dzdt_i - dzdt_f);
-        float coef = cc_expf(-(1.0f * ref));
-        advx = coef * advx;
-        advy = coef * advy;
+        return cc_expf(-(1.0f * ref));
     }
+    return -1.0f;
 }
 
 /* CONMOME (moment.f90:280-780) and, SPH, CONMOME_S (moment.f90:783-1268):
@@ -488,7 +492,7 @@ struct YFace {
 /* CONMOME / CONMOME_S x direction at one face (moment.f90:409-568,
  * 1272-1384); `span`: inside the advection span */
 template <bool SPH>
-__device__ __forceinline__ float conmome_x(const GcLayerDev &L, const XFace &f, int j, int jy, bool span) {
+__device__ __forceinline__ float conmome_x(const GcLayerDev &L, const XFace &f, int j, int jy, bool span, float brk) {
     const float konst = (L.fric_switch != 1) ? 0.5f * L.dt * CC_GRAV : 0.0f;
     const float fm = L.fric_coef;
     float dd = 0.0f, df = 0.0f, ff;
@@ -562,7 +566,10 @@ __device__ __forceinline__ float conmome_x(const GcLayerDev &L, const XFace &f, 
                 advy = ay * (qdiv(f.p_c * xqq, dp1c) - qdiv(f.p_s * xqe, face1(f.d_cs, f.d_ps)));
             }
         }
-        wave_breaking(f.d_c, f.z_c, f.z1_c, L.dt, advx, advy);
+        if (brk >= 0.0f) {
+            advx = brk * advx;
+            advy = brk * advy;
+        }
         xp = xp - advx - advy;
     }
     if (L.fric_switch != 1) xp = fdiv1(xp, 1.0f + ff);
@@ -575,7 +582,8 @@ __device__ __forceinline__ float conmome_x(const GcLayerDev &L, const XFace &f, 
 
 /* CONMOME / CONMOME_S y direction at one face (moment.f90:570-780) */
 template <bool SPH>
-__device__ __forceinline__ float conmome_y(const GcLayerDev &L, const YFace &f, int i, int j, int ix, bool span) {
+__device__ __forceinline__ float conmome_y(const GcLayerDev &L, const YFace &f, int i, int j, int ix, bool span,
+                                           float brk) {
     const float konst = (L.fric_switch != 1) ? 0.5f * L.dt * CC_GRAV : 0.0f;
     const float fm = L.fric_coef;
     float dd = 0.0f, df = 0.0f, ff;
@@ -651,7 +659,10 @@ __device__ __forceinline__ float conmome_y(const GcLayerDev &L, const YFace &f, 
                 advx = bx * (qdiv(f.q_c * xpp, dq1c) - qdiv(f.q_w * xpe, face1(f.d_w, f.d_wq)));
             }
         }
-        wave_breaking(f.d_c, f.z_c, f.z1_c, L.dt, advx, advy);
+        if (brk >= 0.0f) {
+            advx = brk * advx;
+            advy = brk * advy;
+        }
         xq = xq - advx - advy;
     }
     if (L.fric_switch != 1) xq = fdiv1(xq, 1.0f + ff);
@@ -729,7 +740,7 @@ __global__ void k_conmome(GcLayerDev L, int upd) {
             load_x(f, get);
             f.h_c = __ldg(L.h + c); f.h_p = __ldg(L.h + c + 1); f.hp_c = __ldg(L.hp + c);
             f.z1_c = __ldg(L.z1 + c);
-            out = conmome_x<SPH>(L, f, j, jy, span);
+            out = conmome_x<SPH>(L, f, j, jy, span, breaking(f.d_c, f.z_c, f.z1_c, L.dt));
         }
         L.m2[c] = out;
     } else {
@@ -740,7 +751,7 @@ __global__ void k_conmome(GcLayerDev L, int upd) {
             load_y(f, get);
             f.h_c = __ldg(L.h + c); f.h_q = __ldg(L.h + c + P); f.hq_c = __ldg(L.hq + c);
             f.z1_c = __ldg(L.z1 + c);
-            out = conmome_y<SPH>(L, f, i, j, ix, span);
+            out = conmome_y<SPH>(L, f, i, j, ix, span, breaking(f.d_c, f.z_c, f.z1_c, L.dt));
         }
         L.n2[c] = out;
     }
@@ -791,6 +802,7 @@ __device__ __forceinline__ void conmome_tile_body(const GcLayerDev &L, int upd) 
     const bool inx = L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && i <= ix - 2 && j >= 1);
     const bool iny = L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && j >= 1 && j <= jy - 2);
     const float h_c = __ldg(L.h + c), z1_c = __ldg(L.z1 + c);
+    const float brk = span ? breaking(get(0, 0, 0), get(1, 0, 0), z1_c, L.dt) : -1.0f;
     float outx = 0.0f, outy = 0.0f;
     if (inx) {
         XFace f;
@@ -798,7 +810,7 @@ __device__ __forceinline__ void conmome_tile_body(const GcLayerDev &L, int upd) 
         else load_x(f, get);
         f.h_c = h_c; f.h_p = __ldg(L.h + c + 1); f.hp_c = __ldg(L.hp + c);
         f.z1_c = z1_c;
-        outx = conmome_x<SPH>(L, f, j, jy, span);
+        outx = conmome_x<SPH>(L, f, j, jy, span, brk);
     }
     if (iny) {
         YFace f;
@@ -806,7 +818,7 @@ __device__ __forceinline__ void conmome_tile_body(const GcLayerDev &L, int upd) 
         else load_y(f, get);
         f.h_c = h_c; f.h_q = __ldg(L.h + c + P); f.hq_c = __ldg(L.hq + c);
         f.z1_c = z1_c;
-        outy = conmome_y<SPH>(L, f, i, j, ix, span);
+        outy = conmome_y<SPH>(L, f, i, j, ix, span, brk);
     }
     L.m2[c] = outx;
     L.n2[c] = outy;
@@ -1095,6 +1107,250 @@ __global__ void k_mass_c_jnq(GcLayerDev Pl, GcLayerDev L, int ir, int is, int ie
         mass_c_store<NONLIN>(L, c, L.z1[c], L.m1[c], L.m1[c - 1], L.n1[c], L.n1[c - L.pitch], L.h[c]);
     } else {
         mass_c_jnq_edge<NONLIN>(Pl, L, i, j, ir, is, ie, js, je);
+    }
+}
+
+/* JNQ / NEWQ (all_grids.f90:452-801) at one parent cell of a child side: the
+ * flux through it at sub-step t, as k_edges puts it into its profile: the
+ * parent's own at t = 1, else the blend of it with the forecast of the end of
+ * the parent's step.  The forecast is formed at t = 2 (`save`: and cached) and
+ * read from the cache after that, since JNZ changes what it is formed from. */
+struct EdgeArgs {
+    int ir, rel_time, is, ie, js, je, t;
+};
+__device__ __forceinline__ float newq_profile(const GcLayerDev &Pl, const EdgeArgs &E, bool vert, int sd, int line,
+                                              int b, bool save) {
+    const int I = vert ? line : b, J = vert ? b : line;
+    const int Pp = Pl.pitch;
+    const size_t c = (size_t)(J - 1) * Pp + (I - 1);
+    const float own = vert ? Pl.m1[c] : Pl.n1[c];
+    if (E.t == 1) return own;
+    const size_t cn = vert ? c + 1 : c + Pp; /* IP1 or JP1 neighbour */
+    if (!((Pl.h[c] + Pl.z2[c] > CC_GX) && (Pl.h[cn] + Pl.z2[cn] > CC_GX))) return 0.0f;
+    float *cache = vert ? Pl.yflux + (size_t)sd * Pl.ny + (J - 1) : Pl.xflux + (size_t)sd * Pl.nx + (I - 1);
+    float x;
+    if (E.t == 2) {
+        if (Pl.laycord == 0) {
+            if (vert) {
+                const size_t cm = c - Pp; /* JM1 = J-1 */
+                const float tot_n = Pl.n1[c] + Pl.n1[c + 1] + Pl.n1[cm] + Pl.n1[cm + 1];
+                const float r2 = Pl.explicit_r24 ? Pl.r2[c]
+                                 : GC_ROW(Pl, GC_CX, J - 1) * fmaxf(Pl.hp ? Pl.hp[c] :
+                                   ((Pl.h[c] > CC_GX) ? 0.5f * (Pl.h[c] + Pl.h[c + 1]) : 0.0f), 0.0f);
+                x = Pl.m1[c] - r2 * (Pl.z2[c + 1] - Pl.z2[c]) + GC_ROW(Pl, GC_R3, J - 1) * tot_n;
+            } else {
+                const size_t cw = c - 1; /* IM1 = I-1 */
+                const float tot_m = Pl.m1[cw] + Pl.m1[cw + Pp] + Pl.m1[c] + Pl.m1[c + Pp];
+                const float r4 = Pl.explicit_r24 ? Pl.r4[c]
+                                 : GC_ROW(Pl, GC_CY, J - 1) * fmaxf(Pl.hq ? Pl.hq[c] :
+                                   ((Pl.h[c] > CC_GX) ? 0.5f * (Pl.h[c] + Pl.h[c + Pp]) : 0.0f), 0.0f);
+                x = Pl.n1[c] - r4 * (Pl.z2[c + Pp] - Pl.z2[c]) - GC_ROW(Pl, GC_R5, J - 1) * tot_m;
+            }
+        } else if (vert) {
+            const float hm = Pl.hp[c] + 0.5f * (Pl.z2[c] + Pl.z2[c + 1]);
+            x = Pl.m1[c] - Pl.grx * hm * (Pl.z2[c + 1] - Pl.z2[c]);
+        } else {
+            const float hn = Pl.hq[c] + 0.5f * (Pl.z2[c] + Pl.z2[c + Pp]);
+            x = Pl.n1[c] - Pl.gry * hn * (Pl.z2[c + Pp] - Pl.z2[c]);
+        }
+        if (fabsf(x) < CC_EPS) x = 0.0f;
+        if (save) *cache = x;
+    } else {
+        x = *cache;
+    }
+    const float c1 = ((float)E.t - 1.0f) / (float)E.rel_time, c2 = 1.0f - c1;
+    return c1 * x + c2 * own;
+}
+
+/* the child's edge node `run` (1-based along the edge) of side `side`
+ * (0 left M, 1 right M, 2 bottom N, 3 top N) at sub-step t: EDGEINTERP_VERT /
+ * _HORI on that profile, zero where the child is dry.  own: the one thread
+ * that stores the node also caches the forecasts of the node's parent cell. */
+__device__ __forceinline__ float edge_node(const GcLayerDev &Pl, const GcLayerDev &C, const EdgeArgs &E, int side,
+                                           int run, bool own) {
+    const bool vert = side < 2;
+    const int sd = side & 1;
+    const int line = vert ? (sd == 0 ? E.is - 1 : E.ie) : (sd == 0 ? E.js - 1 : E.je);
+    const int a0 = vert ? E.js : E.is, a1 = vert ? E.je : E.ie;
+    const int a = a0 + (run - 1) / E.ir, kk = (run - 1) % E.ir + 1;
+    const float pm = newq_profile(Pl, E, vert, sd, line, a - 1, own && a == a0 && kk == 1);
+    const float p0 = newq_profile(Pl, E, vert, sd, line, a, own && kk == 1);
+    const float pp = newq_profile(Pl, E, vert, sd, line, a + 1, own && a == a1 && kk == E.ir);
+    const float fs = 0.5f * (pm + p0);
+    const float fe = 0.5f * (pp + p0);
+    const float cc1 = (float)((double)(fe - fs) / (double)(2 * E.ir));
+    const float cc2 = -cc1 + fs;
+    const int fixed = vert ? (sd == 0 ? 0 : C.nx - 1) : (sd == 0 ? 0 : C.ny - 1);
+    const size_t cc = vert ? (size_t)run * C.pitch + fixed : (size_t)fixed * C.pitch + run;
+    float val = 2.0f * (float)kk * cc1 + cc2;
+    if (C.h[cc] + C.z1[cc] <= CC_GX) val = 0.0f;
+    return val;
+}
+
+/* CONMASS / CONMASS_S (mass.f90:162-278) of one cell from its fluxes */
+template <bool SPH>
+__device__ __forceinline__ void conmass(const GcLayerDev &L, int j, float z1, float m_c, float m_w, float n_c,
+                                        float n_s, float h, float &z, float &dz) {
+    float zz;
+    bool open;
+    if (SPH) {
+        const float r1 = GC_ROW(L, GC_R1, j), r11 = GC_ROW(L, GC_R11, j);
+        const float r6 = GC_ROW(L, GC_R6, j), r6m = GC_ROW(L, GC_R6, j - 1);
+        zz = z1 - r1 * (m_c - m_w) - r11 * (n_c * r6 - n_s * r6m);
+        open = h >= CC_ELMAX;
+    } else {
+        zz = z1 - L.rx * (m_c - m_w) - L.ry * (n_c - n_s);
+        open = h > CC_ELMAX;
+    }
+    if (fabsf(zz) < CC_EPS) zz = 0.0f;
+    const float dd = zz + h;
+    const bool wet = open && dd >= CC_GX;
+    dz = wet ? dd : 0.0f;
+    z = wet ? zz : -h;
+}
+
+/* One step of a nonlinear layer in one launch: a child's sub-step (JNQ / NEWQ
+ * edge fluxes, CONMASS, CONMOME, UPDATE's edge copy) or a root layer's step
+ * (CONMASS, OPEN, CONMOME and, maxamp, the maximum).  A block of 32 x NL_TY cells
+ * stages M and N of its window (two cells of halo, clamped to the grid) in
+ * shared memory, computes the new surface and total depth of the cells its
+ * faces read (one cell below and west, two above and east: the mass of a halo
+ * cell is computed by every block that reads it), then its cells' faces.  The
+ * separate launches wrote the surface and the depth and read both back, and
+ * each paid a launch on the chain of a sub-step.
+ *
+ * A child's edge fluxes belong to this launch: every thread that reads such a
+ * node computes it (edge_node), and the block that owns it stores it, so
+ * nothing read here is written here.
+ *
+ * Bound by instruction issue and latency (about 1500 warp instructions for 32
+ * cells, half of all cycles issuing), not by memory.  One step, ncu on B200,
+ * separate launches -> this kernel: a 601 x 501 child 24.0 -> 21.2 us; a
+ * 184 x 142 child's sub-step 14.4 -> 8.1 us; a 723 x 603 spherical root
+ * 35.8 -> 26.1 us.
+ *
+ * SPLIT gives the x and y face of a cell to two threads: a small grid leaves
+ * most of the chip idle, and the chain of one cell is what it waits for.  The
+ * line is at two blocks per SM, where every block is resident in both forms;
+ * split against unsplit: 108 blocks 8.1 against 10.8 us, 1197 blocks 21.2
+ * against 21.2, 1748 blocks 28.4 against 26.1. */
+static constexpr int NL_TY = 8;         /* rows of cells per block */
+static constexpr size_t NL_SPLIT = 296; /* blocks up to which SPLIT is taken */
+template <bool SPH, bool ROOT, bool SPLIT>
+__global__ void __launch_bounds__((SPLIT ? 2 : 1) * BX * NL_TY) k_nonlinear_step(GcLayerDev Pl, GcLayerDev L, EdgeArgs E,
+                                                                            int upd, int maxamp) {
+    pdl_enter();
+    constexpr int TY = NL_TY, TW = BX + 4, TH = TY + 4, THREADS = (SPLIT ? 2 : 1) * BX * TY;
+    __shared__ float tile[4][TH][TW]; /* DZ, Z, M, N */
+    const int P = L.pitch, ix = L.nx, jy = L.ny;
+    const int i0 = blockIdx.x * BX, j0 = blockIdx.y * TY;
+    /* the window, and the halo of it that mass reads, lie inside the grid and
+     * off its edges */
+    const bool inside = i0 >= 3 && i0 + TW - 3 <= ix - 2 && j0 >= 3 && j0 + TH - 3 <= jy - 2;
+    for (int t = threadIdx.y * BX + threadIdx.x; t < TW * TH; t += THREADS) {
+        const int tj = t / TW, ti = t - tj * TW;
+        const int i = i0 + ti - 2, j = j0 + tj - 2;
+        if (inside) {
+            const size_t g = (size_t)j * P + i;
+            tile[2][tj][ti] = L.m1[g];
+            tile[3][tj][ti] = L.n1[g];
+        } else {
+            const int ci = min(max(i, 0), ix - 1), cj = min(max(j, 0), jy - 1);
+            const size_t g = (size_t)cj * P + ci;
+            float m, n;
+            if (ROOT) {
+                m = L.m1[g];
+                n = L.n1[g];
+            } else {
+                const bool own = i == ci && j == cj && ti >= 2 && ti < BX + 2 && tj >= 2 && tj < TY + 2;
+                if ((ci == 0 || ci == ix - 1) && cj >= 1) {
+                    m = edge_node(Pl, L, E, ci == 0 ? 0 : 1, cj, own);
+                    if (own) L.m1w[g] = m;
+                } else {
+                    m = L.m1[g];
+                }
+                if ((cj == 0 || cj == jy - 1) && ci >= 1) {
+                    n = edge_node(Pl, L, E, cj == 0 ? 2 : 3, ci, own);
+                    if (own) L.n1w[g] = n;
+                } else {
+                    n = L.n1[g];
+                }
+            }
+            tile[2][tj][ti] = m;
+            tile[3][tj][ti] = n;
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.y * BX + threadIdx.x; t < (TW - 1) * (TH - 1); t += THREADS) {
+        const int tj = t / (TW - 1) + 1, ti = t - (tj - 1) * (TW - 1) + 1;
+        const int i = i0 + ti - 2, j = j0 + tj - 2;
+        const bool own = ti >= 2 && ti < BX + 2 && tj >= 2 && tj < TY + 2 && i < ix && j < jy;
+        const int ci = inside ? i : min(max(i, 0), ix - 1), cj = inside ? j : min(max(j, 0), jy - 1);
+        const size_t g = (size_t)cj * P + ci;
+        float z, dz = 0.0f; /* the total depth of cells without a mass equation is never written: 0 */
+        bool mass = true;
+        if (!inside) mass = ROOT ? (ci >= 1 && ci <= ix - 2 && cj >= 1 && cj <= jy - 2) : (ci >= 1 && cj >= 1);
+        if (mass) {
+            const int si = ci - i0 + 2, sj = cj - j0 + 2;
+            conmass<SPH>(L, cj, L.z1[g], tile[2][sj][si], tile[2][sj][si - 1], tile[3][sj][si], tile[3][sj - 1][si],
+                         L.h[g], z, dz);
+        } else if (ROOT) {
+            z = open_cell(L, ci, cj);
+        } else {
+            z = L.z1[g];
+        }
+        tile[0][tj][ti] = dz;
+        tile[1][tj][ti] = z;
+        if (own) {
+            if (mass) L.dz2[g] = dz;
+            if (mass || ROOT || !upd) L.z2[g] = z;
+            if (ROOT && maxamp) {
+                const float x = L.zmax[g];
+                if (!(x >= z)) L.zmax[g] = z;
+            }
+        }
+    }
+    __syncthreads();
+    /* SPLIT: x faces on the first TY rows of threads, y faces on the others */
+    const bool do_x = !SPLIT || threadIdx.y < TY, do_y = !SPLIT || threadIdx.y >= TY;
+    const int ty = do_x ? threadIdx.y : threadIdx.y - TY;
+    const int i = i0 + threadIdx.x, j = j0 + ty;
+    if (i >= ix || j >= jy) return;
+    const size_t c = (size_t)j * P + i;
+    auto get = [&](int f, int di, int dj) {
+        const int ii = min(max(i + di, 0), ix - 1) - i0 + 2, jj = min(max(j + dj, 0), jy - 1) - j0 + 2;
+        return tile[f][jj][ii];
+    };
+    const float *own = &tile[0][ty + 2][threadIdx.x + 2];
+    auto get_in = [&](int f, int di, int dj) { return own[(f * TH + dj) * TW + di]; };
+    const bool span = adv_span(i, j, ix, jy);
+    const float h_c = __ldg(L.h + c), z1_c = L.z1[c];
+    const float brk = span ? breaking(own[0], own[TH * TW], z1_c, L.dt) : -1.0f;
+    if (do_x) {
+        /* UPDATE's edge copy (all_grids.f90:323-324) */
+        if (!ROOT && upd && (i == 0 || j == 0)) L.z2[c] = get(1, i == 0 ? 1 : 0, j == 0 ? 1 : 0);
+        float out = 0.0f;
+        if (ROOT ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && i <= ix - 2 && j >= 1)) {
+            XFace f;
+            if (inside) load_x(f, get_in);
+            else load_x(f, get);
+            f.h_c = h_c; f.h_p = __ldg(L.h + c + 1); f.hp_c = __ldg(L.hp + c);
+            f.z1_c = z1_c;
+            out = conmome_x<SPH>(L, f, j, jy, span, brk);
+        }
+        L.m2[c] = out;
+    }
+    if (do_y) {
+        float out = 0.0f;
+        if (ROOT ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && j >= 1 && j <= jy - 2)) {
+            YFace f;
+            if (inside) load_y(f, get_in);
+            else load_y(f, get);
+            f.h_c = h_c; f.h_q = __ldg(L.h + c + P); f.hq_c = __ldg(L.hq + c);
+            f.z1_c = z1_c;
+            out = conmome_y<SPH>(L, f, i, j, ix, span, brk);
+        }
+        L.n2[c] = out;
     }
 }
 
@@ -1624,6 +1880,33 @@ bool gc_launch_edges_mass(const GcLayerDev &P, const GcLayerDev &C, int rel_size
     (void)rel_time;
     if (C.laygov == 1) launch(k_mass_c_jnq<true>, grid2(C), dim3(BX, BY), 0, s, P, C, rel_size, is, ie, js, je);
     else launch(k_mass_c_jnq<false>, grid2(C), dim3(BX, BY), 0, s, P, C, rel_size, is, ie, js, je);
+    return true;
+}
+
+template <bool SPH, bool ROOT>
+static void launch_nonlinear(const GcLayerDev &P, const GcLayerDev &L, const EdgeArgs &E, int upd, int maxamp,
+                             cudaStream_t s) {
+    const dim3 grid((unsigned)((L.nx + BX - 1) / BX), (unsigned)((L.ny + NL_TY - 1) / NL_TY), 1);
+    if ((size_t)grid.x * grid.y <= NL_SPLIT)
+        launch(k_nonlinear_step<SPH, ROOT, true>, grid, dim3(BX, 2 * NL_TY), 0, s, P, L, E, upd, maxamp);
+    else
+        launch(k_nonlinear_step<SPH, ROOT, false>, grid, dim3(BX, NL_TY), 0, s, P, L, E, upd, maxamp);
+}
+
+bool gc_launch_child_step(const GcLayerDev &P, const GcLayerDev &C, int rel_size, int rel_time, const int *corners,
+                          int t, cudaStream_t s) {
+    if (C.root || C.laygov != 1) return false;
+    const EdgeArgs E = {rel_size, rel_time, corners[0], corners[1], corners[2], corners[3], t};
+    if (C.laycord == 0) launch_nonlinear<true, false>(P, C, E, 1, 0, s);
+    else launch_nonlinear<false, false>(P, C, E, 1, 0, s);
+    return true;
+}
+
+bool gc_launch_root_step(const GcLayerDev &L, bool maxamp, cudaStream_t s) {
+    if (!L.root || L.laygov != 1) return false;
+    const EdgeArgs E = {1, 1, 0, 0, 0, 0, 1};
+    if (L.laycord == 0) launch_nonlinear<true, true>(L, L, E, 0, maxamp ? 1 : 0, s);
+    else launch_nonlinear<false, true>(L, L, E, 0, maxamp ? 1 : 0, s);
     return true;
 }
 

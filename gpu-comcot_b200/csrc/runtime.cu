@@ -810,6 +810,19 @@ void gc_subcycle(int parent_id) {
             /* edge fluxes and mass: one launch at a Cartesian child's first
              * sub-step (gc_launch_edges_mass), two otherwise */
             int pre = 2;
+            if (!C.has_sc && C.children.empty() &&
+                gc_launch_child_step(P.view(), C.view(), C.rel_size, C.rel_time, C.corners, k, g_rt.stream)) {
+                /* a nonlinear child's whole sub-step */
+                g_rt.launches++;
+                C.z2_valid = C.mn2_valid = true;
+                if (k == nhalf) {
+                    gc_launch_jnz(P.view(), C.view(), C.rel_size, C.rel_time, C.corners, g_rt.stream);
+                    g_rt.launches++;
+                }
+                gc_swap(C);
+                C.sc_stepped = true;
+                continue;
+            }
             if (C.has_sc) {
                 /* EDGE_INTERP_SC / NEWQ_SC (all_grids.f90:996-1364) */
                 const GcLayerDev cv = C.view();
