@@ -445,6 +445,7 @@ __device__ __forceinline__ float face2(float a, float b) {
  * needed to know that it does not. */
 __device__ __forceinline__ float breaking(float dz2c, float z2c, float z1c, float dt) {
     const float a = fabs_(z2c - z1c);
+    if (a == 0.0f) return -1.0f; /* still, or land */
     if (a * a < 0.0063f * (dt * dt) * (CC_GRAV * dz2c)) return -1.0f;
     float cc = sqrtf(CC_GRAV * dz2c);
     float dzdt_f = CC_BRK_F * cc;
@@ -457,243 +458,133 @@ __device__ __forceinline__ float breaking(float dz2c, float z2c, float z1c, floa
     return -1.0f;
 }
 
-/* CONMOME (moment.f90:280-780) and, SPH, CONMOME_S (moment.f90:783-1268):
- * the same structure; the spherical form takes the wet/dry face depth as
- * HP + (Z + Z(I+1))/2, the pressure coefficient R2 / R4 of its row, Coriolis
- * +4 R3 XQQ / -4 R5 XPP, advection coefficients R21 (= R1) / R0 / R22 per
- * row, and applies the y friction to XQ (the Cartesian routine subtracts it
- * from XP, moment.f90:672).
+/* a row's coefficients after those of GcLayerDev::rows: rows2's R0 and R22 */
+constexpr int ROW_R0 = GC_ROWW, ROW_R22 = GC_ROWW + 1, ROW_W = GC_ROWW + 2;
+__device__ __forceinline__ float row_value(const GcLayerDev &L, int j, int k) {
+    return k < GC_ROWW ? GC_ROW(L, k, j) : L.rows2[2 * (size_t)j + k - GC_ROWW];
+}
+
+/* the friction factor konst*FM^2 |flux| / DF^(7/3) of a face, 0 where it can
+ * change no bit of the result: 1 + FF rounds to 1 below 2^-25, and with
+ * `subtract` XP - FF*P rounds to XP where |FF*P| is below 2^-26 |XP|.  The
+ * estimate that decides it is made of the hardware's approximations, off by
+ * 1e-5 at most, and taken 1 % high; a NaN or an XP of 0 takes the exact value.
+ * The root, the power (in double) and the division are two thirds of a face's
+ * instructions where the water is too deep for friction to count. */
+__device__ __forceinline__ float friction(float konst_fm2, float p, float cross, float df, float xp, bool subtract) {
+    const float s = p * p + cross * cross;
+    if (s == 0.0f && df >= CC_DFMIN) return konst_fm2 * s;
+    float root, lg, pw;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(s));
+    asm("lg2.approx.f32 %0, %1;" : "=f"(lg) : "f"(df));
+    asm("ex2.approx.f32 %0, %1;" : "=f"(pw) : "f"(-2.3333333f * lg));
+    const float est = 1.01f * fabsf(konst_fm2) * root * pw;
+    if (est < 0x1p-25f && (!subtract || est * fabsf(p) < 0x1p-26f * fabsf(xp))) return 0.0f;
+    /* df >= DFMIN here unless it is NaN, so the power is positive */
+    const float fnum = konst_fm2 * sqrtf(s);
+    return (fnum == 0.0f && df >= CC_DFMIN) ? fnum : fnum / cc_powf(df, CC_MANNEXP);
+}
+
+/* CONMOME (moment.f90:280-780) and, SPH, CONMOME_S (moment.f90:783-1268) at
+ * one face: X, between (I,J) and (I+1,J), or else between (I,J) and (I,J+1).
+ * The two directions are one routine in the frame of the face, `along` its
+ * normal and `cross` to it, and so are the two Cartesian and spherical ones:
+ * the spherical form takes the wet/dry face depth as HP + (Z + Z(I+1))/2, the
+ * pressure coefficient R2 / R4 of its row, Coriolis +4 R3 XQQ / -4 R5 XPP,
+ * advection coefficients R21 (= R1) / R0 / R22 per row, and applies the y
+ * friction to XQ (the Cartesian routine subtracts it from XP, which is unused,
+ * moment.f90:672).
  *
- * Every value a face can need (its stencil reaches two cells back along the
- * face normal's neighbour axis and one cell forward) is loaded first, as
- * one batch of independent loads at clamped, in-bounds indices; the
- * branches then run on registers.  Clamped indices coincide with the
- * reference's wherever a value is used: the two-back neighbours are read
- * only inside the advection span, whose cells are at least 10 from every
- * edge. */
-/* the stencil of one x face (I,J)-(I+1,J): names give the cell relative to
- * (I,J): p = I+1, m = I-1, p2 = I+2, n = J+1, s = J-1, s2 = J-2; zpn etc.
- * are the surface's corners for the modified-scheme term */
-struct XFace {
-    float h_c, h_p, hp_c, d_c, d_p, d_p2, d_m, d_cn, d_pn, d_cs, d_ps;
-    float z_c, z_p, z1_c, q_c, q_p, q_cs, q_ps, q_cn, q_pn, q_cs2, q_ps2;
-    float p_c, p_p, p_m, p_n, p_s;
-    float z_pn, z_ps, z_cn, z_cs;
-};
-/* the stencil of one y face (I,J)-(I,J+1): q = J+1, q2 = J+2, s = J-1,
- * e = I+1, w = I-1, w2 = I-2 */
-struct YFace {
-    float h_c, h_q, hq_c, d_c, d_q, d_q2, d_s, d_e, d_eq, d_w, d_wq;
-    float z_c, z_q, z1_c, p_c, p_q, p_w, p_wq, p_e, p_eq, p_w2, p_w2q;
-    float q_c, q_q, q_s, q_e, q_w;
-    float z_eq, z_wq, z_e, z_w;
-};
-
-/* CONMOME / CONMOME_S x direction at one face (moment.f90:409-568,
- * 1272-1384); `span`: inside the advection span */
-template <bool SPH>
-__device__ __forceinline__ float conmome_x(const GcLayerDev &L, const XFace &f, int j, int jy, bool span, float brk) {
-    const float konst = (L.fric_switch != 1) ? 0.5f * L.dt * CC_GRAV : 0.0f;
-    const float fm = L.fric_coef;
-    float dd = 0.0f, df = 0.0f, ff;
-    bool noflux = false;
-    if (f.h_c <= CC_ELMAX || f.hp_c <= CC_ELMAX) {
-        noflux = true;
+ * get(field, along, cross) reads DZ2 (0), Z2 (1), M1 (2) or N1 (3) at an offset
+ * from the face's cell, clamped to the grid.  Clamped indices coincide with the
+ * reference's wherever a value is used: the advection terms are formed only in
+ * `span`, at least 10 cells from every edge.
+ *
+ * row(k) is coefficient k of the face's row (GC_* of rows, then rows2).
+ *
+ * The upwind side of each advection term is a choice of offsets, so that one
+ * sequence serves both signs: written as the reference's branches, a warp with
+ * both signs in it went through two sets of loads and divisions, and all the
+ * stencil's values were loaded ahead of them (601 x 501 child 21.2 -> 17.5 us
+ * with this and the tests in friction and breaking). */
+template <bool SPH, bool X, typename Get, typename Row>
+__device__ __forceinline__ float conmome_face(const GcLayerDev &L, const Get &get, const Row &row, int i, int j,
+                                              float h_c, float h_p, float hf, bool span, float brk) {
+    constexpr int F = X ? 2 : 3, G = X ? 3 : 2; /* the face's flux and the other */
+    if (h_c <= CC_ELMAX || hf <= CC_ELMAX) return 0.0f;
+    const float d_c = get(0, 0, 0), d_p = get(0, 1, 0), z_c = get(1, 0, 0), z_p = get(1, 1, 0);
+    const float d1 = face1(d_c, d_p);
+    float dd, df;
+    if (d_c > CC_GX && d_p > CC_GX) {
+        dd = face2(d_c, d_p); df = d1;
+    } else if (d_c > CC_GX && d_p <= CC_GX && h_p + z_c > CC_GX) {
+        dd = SPH ? hf + 0.5f * (z_c + z_p) : 0.5f * d_c; df = dd;
+    } else if (d_c <= CC_GX && d_p > CC_GX && h_c + z_p > CC_GX) {
+        dd = SPH ? hf + 0.5f * (z_c + z_p) : 0.5f * d_p; df = dd;
     } else {
-        if (f.d_c > CC_GX && f.d_p > CC_GX) {
-            dd = face2(f.d_c, f.d_p); df = face1(f.d_c, f.d_p);
-        } else if (f.d_c > CC_GX && f.d_p <= CC_GX && f.h_p + f.z_c > CC_GX) {
-            dd = SPH ? f.hp_c + 0.5f * (f.z_c + f.z_p) : 0.5f * f.d_c; df = dd;
-        } else if (f.d_c <= CC_GX && f.d_p > CC_GX && f.h_c + f.z_p > CC_GX) {
-            dd = SPH ? f.hp_c + 0.5f * (f.z_c + f.z_p) : 0.5f * f.d_p; df = dd;
-        } else {
-            noflux = true;
-        }
-        if (!noflux && dd < CC_GX) noflux = true;
+        return 0.0f;
     }
-    if (noflux) return 0.0f;
+    if (dd < CC_GX) return 0.0f;
     if (df < CC_DFMIN) df = CC_DFMIN;
-    float xqq = 0.25f * (f.q_c + f.q_p + f.q_cs + f.q_ps);
-    if (L.fric_switch != 1) {
-        /* df >= DFMIN here unless it is NaN, so the power is positive */
-        const float fnum = konst * fm * fm * sqrtf(f.p_c * f.p_c + xqq * xqq);
-        ff = (fnum == 0.0f && df >= CC_DFMIN) ? fnum : fnum / cc_powf(df, CC_MANNEXP);
-    } else {
-        ff = 0.0f;
+    const float p = get(F, 0, 0);
+    const float q = 0.25f * (get(G, 0, 0) + get(G, 1, 0) + get(G, 0, -1) + get(G, 1, -1));
+    const float cp = SPH ? row(X ? GC_CX : GC_CY) : (X ? L.grx : L.gry);
+    float x = p - cp * dd * (z_p - z_c);
+    if (L.modscm == 0 && (X ? j + 1 < L.ny : i + 1 < L.nx)) {
+        const float scm = qdiv(cp * dd, 12.0f) * ((get(1, 1, 1) - 2.0f * z_p + get(1, 1, -1)) -
+                                                  (get(1, 0, 1) - 2.0f * z_c + get(1, 0, -1)));
+        x = x - scm;
     }
-    const float cpx = SPH ? GC_ROW(L, GC_CX, j) : L.grx;
-    float xp = f.p_c - cpx * dd * (f.z_p - f.z_c);
-    if (L.modscm == 0 && j + 1 < jy) {
-        float scm = qdiv(cpx * dd, 12.0f) * ((f.z_pn - 2.0f * f.z_p + f.z_ps) - (f.z_cn - 2.0f * f.z_c + f.z_cs));
-        xp = xp - scm;
+    const bool rough = L.fric_switch != 1;
+    float ff = 0.0f;
+    if (rough) {
+        const float konst = 0.5f * L.dt * CC_GRAV, fm = L.fric_coef;
+        ff = friction(konst * fm * fm, p, q, df, x, X || SPH);
+        if (X || SPH) x = x - ff * p;
     }
-    if (L.fric_switch != 1) xp = xp - ff * f.p_c;
-    if (SPH) xp = xp + 4.0f * GC_ROW(L, GC_R3, j) * xqq;
-    const float ax = SPH ? GC_ROW(L, GC_R1, j) : L.rx;   /* R21 = R1 */
-    const float ay = SPH ? L.rows2[2 * (size_t)j] : L.ry; /* R0 */
-    float dp1c = face1(f.d_c, f.d_p);
-    if (L.linchk == 1 && dp1c >= CC_GX && span) {
-        float advx, advy;
-        if (f.p_c < 0.0f) {
-            float dp1p = face1(f.d_p, f.d_p2);
-            if (dp1p < CC_GX || f.d_p < CC_GX)
-                advx = ax * (-(qdiv(f.p_c * f.p_c, dp1c)));
-            else
-                advx = ax * (qdiv(f.p_p * f.p_p, dp1p) - qdiv(f.p_c * f.p_c, dp1c));
-        } else {
-            float dp1m = face1(f.d_m, f.d_c);
-            if (dp1m < CC_GX || f.d_c < CC_GX)
-                advx = ax * (qdiv(f.p_c * f.p_c, dp1c));
-            else
-                advx = ax * (qdiv(f.p_c * f.p_c, dp1c) - qdiv(f.p_m * f.p_m, dp1m));
-        }
-        if (xqq < 0.0f) {
-            if (f.d_cn < CC_GX || f.d_pn < CC_GX) {
-                advy = ay * (-(qdiv(f.p_c * xqq, dp1c)));
-            } else if (face1(f.d_cn, f.d_pn) < CC_GX) {
-                advy = ay * (-(qdiv(f.p_c * xqq, dp1c)));
+    if (SPH) x = X ? x + 4.0f * row(GC_R3) * q : x - 4.0f * row(GC_R5) * q;
+    if (L.linchk == 1 && d1 >= CC_GX && span) {
+        /* R21 is R1 */
+        const float ca = X ? (SPH ? row(GC_R1) : L.rx) : (SPH ? row(ROW_R0) : L.ry);
+        const float cc = X ? (SPH ? row(ROW_R0) : L.ry) : (SPH ? row(ROW_R22) : L.rx);
+        float adva, advc;
+        {
+            const bool up = p < 0.0f;
+            const int o = up ? 1 : -1, k = up ? 1 : 0;
+            const float u_c = qdiv(p * p, d1);
+            const float dk = get(0, k, 0), dn = face1(get(0, o, 0), get(0, up ? 2 : 0, 0)), pn = get(F, o, 0);
+            if (dn < CC_GX || dk < CC_GX) {
+                adva = ca * (up ? -u_c : u_c);
             } else {
-                float xqe = 0.25f * (f.q_cn + f.q_pn + f.q_c + f.q_p);
-                advy = ay * (qdiv(f.p_n * xqe, face1(f.d_cn, f.d_pn)) - qdiv(f.p_c * xqq, dp1c));
+                const float u_n = qdiv(pn * pn, dn);
+                adva = ca * (up ? u_n - u_c : u_c - u_n);
             }
-        } else {
-            if (f.d_cs < CC_GX || f.d_ps < CC_GX) {
-                advy = ay * (qdiv(f.p_c * xqq, dp1c));
-            } else if (face1(f.d_cs, f.d_ps) < CC_GX) {
-                advy = ay * (qdiv(f.p_c * xqq, dp1c));
+        }
+        {
+            const bool up = q < 0.0f;
+            const int o = up ? 1 : -1;
+            const float u_c = qdiv(p * q, d1);
+            const float da = get(0, 0, o), db = get(0, 1, o), dn = face1(da, db);
+            if (da < CC_GX || db < CC_GX || dn < CC_GX) {
+                advc = cc * (up ? -u_c : u_c);
             } else {
-                float xqe = 0.25f * (f.q_cs + f.q_ps + f.q_cs2 + f.q_ps2);
-                advy = ay * (qdiv(f.p_c * xqq, dp1c) - qdiv(f.p_s * xqe, face1(f.d_cs, f.d_ps)));
+                const float qn = 0.25f * (get(G, 0, o) + get(G, 1, o) + get(G, 0, o - 1) + get(G, 1, o - 1));
+                const float u_n = qdiv(get(F, 0, o) * qn, dn);
+                advc = cc * (up ? u_n - u_c : u_c - u_n);
             }
         }
         if (brk >= 0.0f) {
-            advx = brk * advx;
-            advy = brk * advy;
+            adva = brk * adva;
+            advc = brk * advc;
         }
-        xp = xp - advx - advy;
+        x = X ? x - adva - advc : x - advc - adva;
     }
-    if (L.fric_switch != 1) xp = fdiv1(xp, 1.0f + ff);
-    if (fabsf(xp) < CC_EPS) xp = 0.0f;
-    float lim = CC_VLIMIT * dd;
-    if (xp > lim) xp = lim;
-    if (xp < -lim) xp = -lim;
-    return xp;
-}
-
-/* CONMOME / CONMOME_S y direction at one face (moment.f90:570-780) */
-template <bool SPH>
-__device__ __forceinline__ float conmome_y(const GcLayerDev &L, const YFace &f, int i, int j, int ix, bool span,
-                                           float brk) {
-    const float konst = (L.fric_switch != 1) ? 0.5f * L.dt * CC_GRAV : 0.0f;
-    const float fm = L.fric_coef;
-    float dd = 0.0f, df = 0.0f, ff;
-    bool noflux = false;
-    if (f.h_c <= CC_ELMAX || f.hq_c <= CC_ELMAX) {
-        noflux = true;
-    } else {
-        if (f.d_c > CC_GX && f.d_q > CC_GX) {
-            dd = face2(f.d_c, f.d_q); df = face1(f.d_c, f.d_q);
-        } else if (f.d_c > CC_GX && f.d_q <= CC_GX && f.h_q + f.z_c > CC_GX) {
-            dd = SPH ? f.hq_c + 0.5f * (f.z_c + f.z_q) : 0.5f * f.d_c; df = dd;
-        } else if (f.d_c <= CC_GX && f.d_q > CC_GX && f.h_c + f.z_q > CC_GX) {
-            dd = SPH ? f.hq_c + 0.5f * (f.z_c + f.z_q) : 0.5f * f.d_q; df = dd;
-        } else {
-            noflux = true;
-        }
-        if (!noflux && dd < CC_GX) noflux = true;
-    }
-    if (noflux) return 0.0f;
-    if (df < CC_DFMIN) df = CC_DFMIN;
-    float xpp = 0.25f * (f.p_c + f.p_q + f.p_w + f.p_wq);
-    if (L.fric_switch != 1) {
-        /* df >= DFMIN here unless it is NaN, so the power is positive */
-        const float fnum = konst * fm * fm * sqrtf(f.q_c * f.q_c + xpp * xpp);
-        ff = (fnum == 0.0f && df >= CC_DFMIN) ? fnum : fnum / cc_powf(df, CC_MANNEXP);
-    } else {
-        ff = 0.0f;
-    }
-    const float cqy = SPH ? GC_ROW(L, GC_CY, j) : L.gry;
-    float xq = f.q_c - cqy * dd * (f.z_q - f.z_c);
-    if (L.modscm == 0 && i + 1 < ix) {
-        float scm = qdiv(cqy * dd, 12.0f) * ((f.z_eq - 2.0f * f.z_q + f.z_wq) - (f.z_e - 2.0f * f.z_c + f.z_w));
-        xq = xq - scm;
-    }
-    /* CONMOME applies -FF*Q to XP, which is unused (moment.f90:672):
-     * no term on XQ; CONMOME_S applies it to XQ (moment.f90:1150) */
-    if (SPH && L.fric_switch != 1) xq = xq - ff * f.q_c;
-    if (SPH) xq = xq - 4.0f * GC_ROW(L, GC_R5, j) * xpp;
-    const float by = SPH ? L.rows2[2 * (size_t)j] : L.ry;     /* R0 */
-    const float bx = SPH ? L.rows2[2 * (size_t)j + 1] : L.rx; /* R22 */
-    float dq1c = face1(f.d_c, f.d_q);
-    if (L.linchk == 1 && dq1c >= CC_GX && span) {
-        float advx, advy;
-        if (f.q_c < 0.0f) {
-            float dq1q = face1(f.d_q, f.d_q2);
-            if (dq1q < CC_GX || f.d_q < CC_GX)
-                advy = by * (-(qdiv(f.q_c * f.q_c, dq1c)));
-            else
-                advy = by * (qdiv(f.q_q * f.q_q, dq1q) - qdiv(f.q_c * f.q_c, dq1c));
-        } else {
-            float dq1m = face1(f.d_s, f.d_c);
-            if (dq1m < CC_GX || f.d_c < CC_GX)
-                advy = by * (qdiv(f.q_c * f.q_c, dq1c));
-            else
-                advy = by * (qdiv(f.q_c * f.q_c, dq1c) - qdiv(f.q_s * f.q_s, dq1m));
-        }
-        if (xpp < 0.0f) {
-            if (f.d_e < CC_GX || f.d_eq < CC_GX) {
-                advx = bx * (-(qdiv(f.q_c * xpp, dq1c)));
-            } else if (face1(f.d_e, f.d_eq) < CC_GX) {
-                advx = bx * (-(qdiv(f.q_c * xpp, dq1c)));
-            } else {
-                float xpe = 0.25f * (f.p_e + f.p_eq + f.p_c + f.p_q);
-                advx = bx * (qdiv(f.q_e * xpe, face1(f.d_e, f.d_eq)) - qdiv(f.q_c * xpp, dq1c));
-            }
-        } else {
-            if (f.d_w < CC_GX || f.d_wq < CC_GX) {
-                advx = bx * (qdiv(f.q_c * xpp, dq1c));
-            } else if (face1(f.d_w, f.d_wq) < CC_GX) {
-                advx = bx * (qdiv(f.q_c * xpp, dq1c));
-            } else {
-                float xpe = 0.25f * (f.p_w + f.p_wq + f.p_w2 + f.p_w2q);
-                advx = bx * (qdiv(f.q_c * xpp, dq1c) - qdiv(f.q_w * xpe, face1(f.d_w, f.d_wq)));
-            }
-        }
-        if (brk >= 0.0f) {
-            advx = brk * advx;
-            advy = brk * advy;
-        }
-        xq = xq - advx - advy;
-    }
-    if (L.fric_switch != 1) xq = fdiv1(xq, 1.0f + ff);
-    if (fabsf(xq) < CC_EPS) xq = 0.0f;
-    float lim = CC_VLIMIT * dd;
-    if (xq > lim) xq = lim;
-    if (xq < -lim) xq = -lim;
-    return xq;
-}
-
-/* a face's stencil from a field accessor get(field, di, dj), di/dj relative
- * to the face's cell; the accessor clamps to the grid */
-template <typename Get>
-__device__ __forceinline__ void load_x(XFace &f, const Get &get) {
-    f.d_c = get(0, 0, 0); f.d_p = get(0, 1, 0); f.d_p2 = get(0, 2, 0); f.d_m = get(0, -1, 0);
-    f.d_cn = get(0, 0, 1); f.d_pn = get(0, 1, 1); f.d_cs = get(0, 0, -1); f.d_ps = get(0, 1, -1);
-    f.z_c = get(1, 0, 0); f.z_p = get(1, 1, 0);
-    f.z_pn = get(1, 1, 1); f.z_ps = get(1, 1, -1); f.z_cn = get(1, 0, 1); f.z_cs = get(1, 0, -1);
-    f.q_c = get(3, 0, 0); f.q_p = get(3, 1, 0); f.q_cs = get(3, 0, -1); f.q_ps = get(3, 1, -1);
-    f.q_cn = get(3, 0, 1); f.q_pn = get(3, 1, 1); f.q_cs2 = get(3, 0, -2); f.q_ps2 = get(3, 1, -2);
-    f.p_c = get(2, 0, 0); f.p_p = get(2, 1, 0); f.p_m = get(2, -1, 0); f.p_n = get(2, 0, 1); f.p_s = get(2, 0, -1);
-}
-template <typename Get>
-__device__ __forceinline__ void load_y(YFace &f, const Get &get) {
-    f.d_c = get(0, 0, 0); f.d_q = get(0, 0, 1); f.d_q2 = get(0, 0, 2); f.d_s = get(0, 0, -1);
-    f.d_e = get(0, 1, 0); f.d_eq = get(0, 1, 1); f.d_w = get(0, -1, 0); f.d_wq = get(0, -1, 1);
-    f.z_c = get(1, 0, 0); f.z_q = get(1, 0, 1);
-    f.z_eq = get(1, 1, 1); f.z_wq = get(1, -1, 1); f.z_e = get(1, 1, 0); f.z_w = get(1, -1, 0);
-    f.p_c = get(2, 0, 0); f.p_q = get(2, 0, 1); f.p_w = get(2, -1, 0); f.p_wq = get(2, -1, 1);
-    f.p_e = get(2, 1, 0); f.p_eq = get(2, 1, 1); f.p_w2 = get(2, -2, 0); f.p_w2q = get(2, -2, 1);
-    f.q_c = get(3, 0, 0); f.q_q = get(3, 0, 1); f.q_s = get(3, 0, -1); f.q_e = get(3, 1, 0); f.q_w = get(3, -1, 0);
+    if (rough) x = fdiv1(x, 1.0f + ff);
+    if (fabsf(x) < CC_EPS) x = 0.0f;
+    const float lim = CC_VLIMIT * dd;
+    if (x > lim) x = lim;
+    if (x < -lim) x = -lim;
+    return x;
 }
 
 /* Fortran spans: I > 10 .AND. I < IX-10 with I = i+1 */
@@ -731,28 +622,19 @@ __global__ void k_conmome(GcLayerDev L, int upd) {
         const int ii = min(max(i + di, 0), ix - 1), jj = min(max(j + dj, 0), jy - 1);
         return __ldg(fields[f] + (size_t)jj * P + ii);
     };
+    auto get_y = [&](int f, int along, int cross) { return get(f, cross, along); };
+    auto row = [&](int k) { return row_value(L, j, k); };
     const bool span = adv_span(i, j, ix, jy);
+    const float h_c = __ldg(L.h + c);
+    const float brk = span ? breaking(get(0, 0, 0), get(1, 0, 0), __ldg(L.z1 + c), L.dt) : -1.0f;
+    float out = 0.0f;
     if (blockIdx.z == 0) {
-        const bool inx = L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && i <= ix - 2 && j >= 1);
-        float out = 0.0f;
-        if (inx) {
-            XFace f;
-            load_x(f, get);
-            f.h_c = __ldg(L.h + c); f.h_p = __ldg(L.h + c + 1); f.hp_c = __ldg(L.hp + c);
-            f.z1_c = __ldg(L.z1 + c);
-            out = conmome_x<SPH>(L, f, j, jy, span, breaking(f.d_c, f.z_c, f.z1_c, L.dt));
-        }
+        if (L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && i <= ix - 2 && j >= 1))
+            out = conmome_face<SPH, true>(L, get, row, i, j, h_c, __ldg(L.h + c + 1), __ldg(L.hp + c), span, brk);
         L.m2[c] = out;
     } else {
-        const bool iny = L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && j >= 1 && j <= jy - 2);
-        float out = 0.0f;
-        if (iny) {
-            YFace f;
-            load_y(f, get);
-            f.h_c = __ldg(L.h + c); f.h_q = __ldg(L.h + c + P); f.hq_c = __ldg(L.hq + c);
-            f.z1_c = __ldg(L.z1 + c);
-            out = conmome_y<SPH>(L, f, i, j, ix, span, breaking(f.d_c, f.z_c, f.z1_c, L.dt));
-        }
+        if (L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && j >= 1 && j <= jy - 2))
+            out = conmome_face<SPH, false>(L, get_y, row, i, j, h_c, __ldg(L.h + c + P), __ldg(L.hq + c), span, brk);
         L.n2[c] = out;
     }
 }
@@ -787,39 +669,20 @@ __device__ __forceinline__ void conmome_tile_body(const GcLayerDev &L, int upd) 
         if (j == 0) L.z2[i] = L.z2[(size_t)P + (i == 0 ? 1 : i)];
         else if (i == 0) L.z2[c] = L.z2[c + 1];
     }
-    /* the tile holds the clamped neighbour of every in-grid cell it covers;
-     * for a cell near the grid edge the clamp is repeated on the offset.  A
-     * block whose window lies inside the grid clamps nothing: its cells read
-     * the tile at fixed offsets from their own slot. */
-    auto get = [&](int f, int di, int dj) {
-        const int ii = min(max(i + di, 0), ix - 1) - i0 + 2, jj = min(max(j + dj, 0), jy - 1) - j0 + 2;
-        return tile[f][jj][ii];
-    };
+    /* the window was staged at clamped indices: every offset from an in-grid
+     * cell holds the clamped neighbour */
     const float *own = &tile[0][threadIdx.y + 2][threadIdx.x + 2];
-    auto get_in = [&](int f, int di, int dj) { return own[(f * TH + dj) * TW + di]; };
-    const bool inside = i0 >= 2 && i0 + TW - 3 <= ix - 1 && j0 >= 2 && j0 + TH - 3 <= jy - 1;
+    auto get = [&](int f, int di, int dj) { return own[(f * TH + dj) * TW + di]; };
+    auto get_y = [&](int f, int along, int cross) { return own[(f * TH + along) * TW + cross]; };
+    auto row = [&](int k) { return row_value(L, j, k); };
     const bool span = adv_span(i, j, ix, jy);
     const bool inx = L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && i <= ix - 2 && j >= 1);
     const bool iny = L.root ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && j >= 1 && j <= jy - 2);
-    const float h_c = __ldg(L.h + c), z1_c = __ldg(L.z1 + c);
-    const float brk = span ? breaking(get(0, 0, 0), get(1, 0, 0), z1_c, L.dt) : -1.0f;
+    const float h_c = __ldg(L.h + c);
+    const float brk = span ? breaking(get(0, 0, 0), get(1, 0, 0), __ldg(L.z1 + c), L.dt) : -1.0f;
     float outx = 0.0f, outy = 0.0f;
-    if (inx) {
-        XFace f;
-        if (inside) load_x(f, get_in);
-        else load_x(f, get);
-        f.h_c = h_c; f.h_p = __ldg(L.h + c + 1); f.hp_c = __ldg(L.hp + c);
-        f.z1_c = z1_c;
-        outx = conmome_x<SPH>(L, f, j, jy, span, brk);
-    }
-    if (iny) {
-        YFace f;
-        if (inside) load_y(f, get_in);
-        else load_y(f, get);
-        f.h_c = h_c; f.h_q = __ldg(L.h + c + P); f.hq_c = __ldg(L.hq + c);
-        f.z1_c = z1_c;
-        outy = conmome_y<SPH>(L, f, i, j, ix, span, brk);
-    }
+    if (inx) outx = conmome_face<SPH, true>(L, get, row, i, j, h_c, __ldg(L.h + c + 1), __ldg(L.hp + c), span, brk);
+    if (iny) outy = conmome_face<SPH, false>(L, get_y, row, i, j, h_c, __ldg(L.h + c + P), __ldg(L.hq + c), span, brk);
     L.m2[c] = outx;
     L.n2[c] = outy;
 }
@@ -1187,16 +1050,16 @@ __device__ __forceinline__ float edge_node(const GcLayerDev &Pl, const GcLayerDe
     return val;
 }
 
-/* CONMASS / CONMASS_S (mass.f90:162-278) of one cell from its fluxes */
+/* CONMASS / CONMASS_S (mass.f90:162-278) of one cell from its fluxes; `row`:
+ * its row's coefficients, the row before it ROW_W earlier */
 template <bool SPH>
-__device__ __forceinline__ void conmass(const GcLayerDev &L, int j, float z1, float m_c, float m_w, float n_c,
+__device__ __forceinline__ void conmass(const GcLayerDev &L, const float *row, float z1, float m_c, float m_w, float n_c,
                                         float n_s, float h, float &z, float &dz) {
     float zz;
     bool open;
     if (SPH) {
-        const float r1 = GC_ROW(L, GC_R1, j), r11 = GC_ROW(L, GC_R11, j);
-        const float r6 = GC_ROW(L, GC_R6, j), r6m = GC_ROW(L, GC_R6, j - 1);
-        zz = z1 - r1 * (m_c - m_w) - r11 * (n_c * r6 - n_s * r6m);
+        const float r6 = row[GC_R6], r6m = row[GC_R6 - ROW_W];
+        zz = z1 - row[GC_R1] * (m_c - m_w) - row[GC_R11] * (n_c * r6 - n_s * r6m);
         open = h >= CC_ELMAX;
     } else {
         zz = z1 - L.rx * (m_c - m_w) - L.ry * (n_c - n_s);
@@ -1223,17 +1086,19 @@ __device__ __forceinline__ void conmass(const GcLayerDev &L, int j, float z1, fl
  * node computes it (edge_node), and the block that owns it stores it, so
  * nothing read here is written here.
  *
- * Bound by instruction issue and latency (about 1500 warp instructions for 32
- * cells, half of all cycles issuing), not by memory.  One step, ncu on B200,
- * separate launches -> this kernel: a 601 x 501 child 24.0 -> 21.2 us; a
- * 184 x 142 child's sub-step 14.4 -> 8.1 us; a 723 x 603 spherical root
- * 35.8 -> 26.1 us.
+ * Bound by instruction issue (about 1050 warp instructions for 32 Cartesian
+ * cells; three of four cycles issue while blocks are resident), not by memory.
+ * One step, ncu on B200, separate launches -> this kernel: a 601 x 501 child
+ * 24.0 -> 17.5 us; a 184 x 142 child's sub-step 14.4 -> 7.5 us; a 723 x 603
+ * spherical root 35.8 -> 21.4 us.  Blocks of 32 x 16 cells, with less halo,
+ * take 19.2, 8.3 and 21.7 us; of 32 x 4, more.
  *
  * SPLIT gives the x and y face of a cell to two threads: a small grid leaves
  * most of the chip idle, and the chain of one cell is what it waits for.  The
  * line is at two blocks per SM, where every block is resident in both forms;
- * split against unsplit: 108 blocks 8.1 against 10.8 us, 1197 blocks 21.2
- * against 21.2, 1748 blocks 28.4 against 26.1. */
+ * split against unsplit, when a face still cost 1.4 times as much: 108 blocks
+ * 8.1 against 10.8 us, 1197 blocks 21.2 against 21.2, 1748 blocks 28.4
+ * against 26.1. */
 static constexpr int NL_TY = 8;         /* rows of cells per block */
 static constexpr size_t NL_SPLIT = 296; /* blocks up to which SPLIT is taken */
 template <bool SPH, bool ROOT, bool SPLIT>
@@ -1242,8 +1107,14 @@ __global__ void __launch_bounds__((SPLIT ? 2 : 1) * BX * NL_TY) k_nonlinear_step
     pdl_enter();
     constexpr int TY = NL_TY, TW = BX + 4, TH = TY + 4, THREADS = (SPLIT ? 2 : 1) * BX * TY;
     __shared__ float tile[4][TH][TW]; /* DZ, Z, M, N */
+    __shared__ float rows[SPH ? TH : 1][ROW_W];
     const int P = L.pitch, ix = L.nx, jy = L.ny;
     const int i0 = blockIdx.x * BX, j0 = blockIdx.y * TY;
+    if (SPH) {
+        const int t = threadIdx.y * BX + threadIdx.x, tj = t / ROW_W;
+        static_assert(TH * ROW_W <= BX * TY, "one coefficient per thread");
+        if (tj < TH) rows[tj][t - tj * ROW_W] = row_value(L, min(max(j0 + tj - 2, 0), jy - 1), t - tj * ROW_W);
+    }
     /* the window, and the halo of it that mass reads, lie inside the grid and
      * off its edges */
     const bool inside = i0 >= 3 && i0 + TW - 3 <= ix - 2 && j0 >= 3 && j0 + TH - 3 <= jy - 2;
@@ -1292,7 +1163,7 @@ __global__ void __launch_bounds__((SPLIT ? 2 : 1) * BX * NL_TY) k_nonlinear_step
         if (!inside) mass = ROOT ? (ci >= 1 && ci <= ix - 2 && cj >= 1 && cj <= jy - 2) : (ci >= 1 && cj >= 1);
         if (mass) {
             const int si = ci - i0 + 2, sj = cj - j0 + 2;
-            conmass<SPH>(L, cj, L.z1[g], tile[2][sj][si], tile[2][sj][si - 1], tile[3][sj][si], tile[3][sj - 1][si],
+            conmass<SPH>(L, rows[SPH ? sj : 0], L.z1[g], tile[2][sj][si], tile[2][sj][si - 1], tile[3][sj][si], tile[3][sj - 1][si],
                          L.h[g], z, dz);
         } else if (ROOT) {
             z = open_cell(L, ci, cj);
@@ -1317,39 +1188,27 @@ __global__ void __launch_bounds__((SPLIT ? 2 : 1) * BX * NL_TY) k_nonlinear_step
     const int i = i0 + threadIdx.x, j = j0 + ty;
     if (i >= ix || j >= jy) return;
     const size_t c = (size_t)j * P + i;
-    auto get = [&](int f, int di, int dj) {
-        const int ii = min(max(i + di, 0), ix - 1) - i0 + 2, jj = min(max(j + dj, 0), jy - 1) - j0 + 2;
-        return tile[f][jj][ii];
-    };
+    /* DZ and Z are there one cell below and west, M and N two, all at clamped
+     * indices */
     const float *own = &tile[0][ty + 2][threadIdx.x + 2];
-    auto get_in = [&](int f, int di, int dj) { return own[(f * TH + dj) * TW + di]; };
+    auto get = [&](int f, int di, int dj) { return own[(f * TH + dj) * TW + di]; };
+    auto get_y = [&](int f, int along, int cross) { return own[(f * TH + along) * TW + cross]; };
+    auto row = [&](int k) { return rows[SPH ? ty + 2 : 0][k]; };
     const bool span = adv_span(i, j, ix, jy);
-    const float h_c = __ldg(L.h + c), z1_c = L.z1[c];
-    const float brk = span ? breaking(own[0], own[TH * TW], z1_c, L.dt) : -1.0f;
+    const float h_c = __ldg(L.h + c);
+    const float brk = span ? breaking(own[0], own[TH * TW], L.z1[c], L.dt) : -1.0f;
     if (do_x) {
         /* UPDATE's edge copy (all_grids.f90:323-324) */
         if (!ROOT && upd && (i == 0 || j == 0)) L.z2[c] = get(1, i == 0 ? 1 : 0, j == 0 ? 1 : 0);
         float out = 0.0f;
-        if (ROOT ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && i <= ix - 2 && j >= 1)) {
-            XFace f;
-            if (inside) load_x(f, get_in);
-            else load_x(f, get);
-            f.h_c = h_c; f.h_p = __ldg(L.h + c + 1); f.hp_c = __ldg(L.hp + c);
-            f.z1_c = z1_c;
-            out = conmome_x<SPH>(L, f, j, jy, span, brk);
-        }
+        if (ROOT ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && i <= ix - 2 && j >= 1))
+            out = conmome_face<SPH, true>(L, get, row, i, j, h_c, __ldg(L.h + c + 1), __ldg(L.hp + c), span, brk);
         L.m2[c] = out;
     }
     if (do_y) {
         float out = 0.0f;
-        if (ROOT ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && j >= 1 && j <= jy - 2)) {
-            YFace f;
-            if (inside) load_y(f, get_in);
-            else load_y(f, get);
-            f.h_c = h_c; f.h_q = __ldg(L.h + c + P); f.hq_c = __ldg(L.hq + c);
-            f.z1_c = z1_c;
-            out = conmome_y<SPH>(L, f, i, j, ix, span, brk);
-        }
+        if (ROOT ? (i <= ix - 2 && j <= jy - 2) : (i >= 1 && j >= 1 && j <= jy - 2))
+            out = conmome_face<SPH, false>(L, get_y, row, i, j, h_c, __ldg(L.h + c + P), __ldg(L.hq + c), span, brk);
         L.n2[c] = out;
     }
 }

@@ -78,3 +78,34 @@ def test_root(oracle_mod, nx, ny, maxamp):
     ref = o.layer(0)
     for f in ("z", "m", "n") + (("zmax",) if maxamp else ()):
         _same(got[f], ref[f], f)
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+@pytest.mark.parametrize("fric", [0.025, 0.0, 1.0e-4])
+def test_friction_lines(oracle_mod, seed, fric):
+    """depths and surfaces spread over many decades put friction on both sides
+    of the sizes below which it is left out, at every face"""
+    nx, ny = 131, 75
+    case = synth.single_layer_case("f", nx, ny, 2.0, 2.0, 0, seed=seed, n_seamounts=0, shelf_cols=0, land_cols=0,
+                                   ngauges=0, laygov=1, fric=fric)
+    L = case.root
+    rng = np.random.default_rng(seed)
+    jj, ii = np.mgrid[0:ny, 0:nx]
+    L.H = (10.0 ** (0.85 + 2.85 * np.sin(ii * 0.11 + seed) * np.cos(jj * 0.13))
+           * rng.uniform(0.7, 1.4, size=(ny, nx))).astype(np.float32)
+    L.hp, L.hq = synth.pc.pq_depth(L.H)
+    L.Z0 = (np.minimum(L.H, 3.0) * 0.5 * 10.0 ** rng.uniform(-7, 0, size=(ny, nx))
+            * np.where(rng.uniform(size=(ny, nx)) < 0.5, -1, 1)).astype(np.float32)
+    s = ReferenceSession(case, fusion=True)
+    try:
+        for _ in range(6):
+            s.step(maxamp=True)
+        got = {"z": s.getz(1), "m": s.getmn(1)[0], "n": s.getmn(1)[1]}
+    finally:
+        s.close()
+    o = oracle_mod.OracleRun(case)
+    o.run(6)
+    ref = o.layer(0)
+    assert np.isfinite(ref["m"]).all()
+    for f in ("z", "m", "n"):
+        _same(got[f], ref[f], f)
