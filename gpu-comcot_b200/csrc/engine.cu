@@ -82,6 +82,7 @@ struct EngMember {
     float *cz[2] = {nullptr, nullptr}, *cm[2] = {nullptr, nullptr}, *cn[2] = {nullptr, nullptr};
     float *cdz2 = nullptr, *xflux = nullptr, *yflux = nullptr;
     int *glayer = nullptr;
+    int ng_child = 0; /* gauges on the child */
     /* SC_OPTION = 1: the outer grid's band forecast of NEWQ_SC (the fused
      * step has written the outer grid's real level 2 by then) */
     float *sm2 = nullptr, *sn2 = nullptr;
@@ -307,11 +308,30 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
         e->launches++;
     }
     cc ^= 1;
+    /* the outer window's momentum and outputs (joined by `s` from ev_cjoin).
+     * JNZ gives the outer grid its final surface at sub-step nhalf, and what
+     * the later sub-steps read of the outer grid is that, the level-1 fluxes
+     * and the cached forecasts: the two go beside them on the other stream.
+     * A 481 x 401 grid whose 184 x 142 child takes three sub-steps:
+     * 33.7 -> 32.4 us a step. */
+    auto window = [&] {
+        cudaEventRecord(e->ev_cfork[a], s);
+        cudaStreamWaitEvent(cs, e->ev_cfork[a], 0);
+        gc_launch_momt_s_window(P, C.corners[0] - 2, C.corners[1] - 1, C.corners[2] - 2, C.corners[3] - 1, cs);
+        gc_launch_step_outputs(P, d_base, step_off, M.step0, flags, 1, M.thr, M.ng, M.gij, M.gw, M.glayer,
+                               M.cz[cc], C.cpitch, M.ts, M.nsteps, win, cs);
+        cudaEventRecord(e->ev_cjoin[a], cs);
+        e->launches += 2;
+    };
+    const bool early = !fb && !C.has_sc && nhalf < C.rel_time;
     for (int t = 2; t <= C.rel_time; t++) {
         const GcLayerDev Cv = child_view(C, M, cc);
         if (!C.has_sc && gc_launch_child_step(P, Cv, C.rel_size, C.rel_time, C.corners, t, s)) {
             e->launches++;
-            if (t == nhalf) jnz(Cv);
+            if (t == nhalf) {
+                jnz(Cv);
+                if (early) window();
+            }
             cc ^= 1;
             continue;
         }
@@ -333,7 +353,10 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
              * which JNZ never reads (its blocks start at child index 1), so
              * it may precede JNZ */
             e->launches += 2 + gc_launch_moment_update(Cv, s);
-            if (t == nhalf) jnz(Cv);
+            if (t == nhalf) {
+                jnz(Cv);
+                if (early) window();
+            }
         }
         cc ^= 1;
     }
@@ -348,14 +371,23 @@ static void eng_nested_step(gc_engine *e, EngMember &M, int local, const int *d_
         e->launches += 2; /* the fused step, the feedback */
         return;
     }
-    cudaEventRecord(e->ev_cfork[a], s);
-    cudaStreamWaitEvent(cs, e->ev_cfork[a], 0);
-    gc_launch_step_outputs(P, d_base, step_off, M.step0, flags, M.thr, M.ng, M.gij, M.gw, M.glayer, M.cz[cc],
-                           C.cpitch, M.ts, M.nsteps, win, cs);
-    cudaEventRecord(e->ev_cjoin[a], cs);
-    gc_launch_momt_s_window(P, C.corners[0] - 2, C.corners[1] - 1, C.corners[2] - 2, C.corners[3] - 1, s);
+    e->launches++; /* the outer step */
+    if (early) {
+        if (M.ng_child > 0) {
+            gc_launch_step_outputs(P, d_base, step_off, M.step0, flags, 2, M.thr, M.ng, M.gij, M.gw, M.glayer,
+                                   M.cz[cc], C.cpitch, M.ts, M.nsteps, win, s);
+            e->launches++;
+        }
+    } else {
+        cudaEventRecord(e->ev_cfork[a], s);
+        cudaStreamWaitEvent(cs, e->ev_cfork[a], 0);
+        gc_launch_step_outputs(P, d_base, step_off, M.step0, flags, 3, M.thr, M.ng, M.gij, M.gw, M.glayer, M.cz[cc],
+                               C.cpitch, M.ts, M.nsteps, win, cs);
+        cudaEventRecord(e->ev_cjoin[a], cs);
+        gc_launch_momt_s_window(P, C.corners[0] - 2, C.corners[1] - 1, C.corners[2] - 2, C.corners[3] - 1, s);
+        e->launches += 2;
+    }
     cudaStreamWaitEvent(s, e->ev_cjoin[a], 0);
-    e->launches += 3; /* the fused step, the window's momentum, the outputs */
 }
 
 /* issues `count` consecutive steps, the first being host step e->gstep + 1
@@ -876,7 +908,10 @@ static int eng_add_member(gc_engine *e, int cls, const float *z0, const float *c
         if (ngauges > 0) {
             std::vector<int> gl((size_t)ngauges, 0);
             if (glayer)
-                for (int g = 0; g < ngauges; g++) gl[g] = glayer[g];
+                for (int g = 0; g < ngauges; g++) {
+                    gl[g] = glayer[g];
+                    M.ng_child += glayer[g] != 0;
+                }
             GC_CUDA_OR_RET(cudaMemcpyAsync(M.glayer, gl.data(), gl.size() * sizeof(int), cudaMemcpyHostToDevice,
                                            e->stream));
             /* the pageable copy is staged before return, but keep `gl` alive until it ran */

@@ -154,8 +154,9 @@ void gc_launch_arrival(const GcLayerDev &L, int step, float thr, cudaStream_t s)
 void gc_launch_gauges(const GcLayerDev &L, int ng, const int *d_ij, float *d_out, cudaStream_t s);
 /* max-eta (flags & 1), arrival (flags & 2) and gauge samples after one outer
  * step of a batched nested member; step = step_off + *step_base; max/arrival
- * over the 0-based window win = {i0, i1, j0, j1} (NULL: the whole layer) */
-void gc_launch_step_outputs(const GcLayerDev &L, const int *step_base, int step_off, int step0, int flags,
+ * over the 0-based window win = {i0, i1, j0, j1} (NULL: the whole layer).
+ * which: 1 the layer's own outputs, 2 the gauges on its child, 3 both */
+void gc_launch_step_outputs(const GcLayerDev &L, const int *step_base, int step_off, int step0, int flags, int which,
                             float thr, int ng, const int *gij, const float *gw, const int *glayer,
                             const float *cz, int cpitch, float *ts, int ts_len, const int *win, cudaStream_t s);
 /* JNZ (window `corners`, 1-based IS, IE, JS, JE), the linear spherical

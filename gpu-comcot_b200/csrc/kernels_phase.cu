@@ -1477,7 +1477,7 @@ __global__ void k_gauges(GcLayerDev L, int ng, const int *ij, float *out) {
  * from the outer layer or the child (cz, pitch cpitch).  The step number is
  * step_off + *step_base (step_base may be NULL), so a replayed graph numbers
  * the steps correctly; step - step0 is the member's 0-based step index. */
-__global__ void k_step_outputs(GcLayerDev L, const int *step_base, int step_off, int step0, int flags,
+__global__ void k_step_outputs(GcLayerDev L, const int *step_base, int step_off, int step0, int flags, int which,
                                float thr, int ng, const int *gij, const float *gw, const int *glayer,
                                const float *cz, int cpitch, float *ts, int ts_len, int wi0, int wj0, int wni,
                                int wnj) {
@@ -1487,6 +1487,7 @@ __global__ void k_step_outputs(GcLayerDev L, const int *step_base, int step_off,
     if (blockIdx.x == 0 && blockIdx.y == 0 && ng > 0) {
         for (int g = threadIdx.y * BX + threadIdx.x; g < ng; g += BX * BY) {
             const bool child = glayer && glayer[g] != 0;
+            if (!(which & (child ? 2 : 1))) continue;
             const float *z = child ? cz : L.z2;
             const size_t P = child ? (size_t)cpitch : (size_t)L.pitch;
             size_t c = (size_t)(gij[2 * g + 1] - 1) * P + (size_t)(gij[2 * g] - 1);
@@ -1499,6 +1500,7 @@ __global__ void k_step_outputs(GcLayerDev L, const int *step_base, int step_off,
             ts[(size_t)local * ng + g] = a + b + d + e;
         }
     }
+    if (!(which & 1)) return;
     int i = wi0 + blockIdx.x * BX + threadIdx.x;
     int j = wj0 + blockIdx.y * BY + threadIdx.y;
     if (i >= wi0 + wni || j >= wj0 + wnj || i >= L.nx || j >= L.ny) return;
@@ -1836,13 +1838,14 @@ void gc_launch_gauges(const GcLayerDev &L, int ng, const int *d_ij, float *d_out
     launch(k_gauges, (ng + 127) / 128, 128, 0, s, L, ng, d_ij, d_out);
 }
 
-void gc_launch_step_outputs(const GcLayerDev &L, const int *step_base, int step_off, int step0, int flags,
+void gc_launch_step_outputs(const GcLayerDev &L, const int *step_base, int step_off, int step0, int flags, int which,
                             float thr, int ng, const int *gij, const float *gw, const int *glayer,
                             const float *cz, int cpitch, float *ts, int ts_len, const int *win, cudaStream_t s) {
     int i0 = 0, j0 = 0, ni = L.nx, nj = L.ny;
     if (win) { i0 = win[0]; ni = win[1] - win[0] + 1; j0 = win[2]; nj = win[3] - win[2] + 1; }
     dim3 grid((unsigned)((ni + BX - 1) / BX), (unsigned)((nj + BY - 1) / BY), 1);
-    launch(k_step_outputs, grid, dim3(BX, BY), 0, s, L, step_base, step_off, step0, flags, thr, ng, gij, gw, glayer,
+    if (!(which & 1)) grid = dim3(1, 1, 1);
+    launch(k_step_outputs, grid, dim3(BX, BY), 0, s, L, step_base, step_off, step0, flags, which, thr, ng, gij, gw, glayer,
                                                  cz, cpitch, ts, ts_len, i0, j0, ni, nj);
 }
 

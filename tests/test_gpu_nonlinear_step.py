@@ -109,3 +109,31 @@ def test_friction_lines(oracle_mod, seed, fric):
     assert np.isfinite(ref["m"]).all()
     for f in ("z", "m", "n"):
         _same(got[f], ref[f], f)
+
+
+@pytest.mark.parametrize("rel_time", [3, 4, 5])
+@pytest.mark.parametrize("laygov", [0, 1])
+@pytest.mark.parametrize("graphs", [0, 1])
+def test_outer_window_beside_later_sub_steps(oracle_mod, rel_time, laygov, graphs):
+    """sub-steps after the feedback run beside the outer window's momentum and
+    outputs; gauges on the child are sampled after the last one"""
+    from comcot_b200.engine import Engine
+    case = synth.nested_case("w", 97, 81, 2.0, 2.0, [60, 79, 30, 49], 3, 30, seed=9, rel_time=rel_time,
+                             child_laygov=laygov, ngauges=2)
+    P, C = case.layers
+    _steep(C, 6, 0.5)
+    case.gauges += [(C.id, 12, 20, 0.4, 0.7), (C.id, 40, 33, 0.1, 0.2), (P.id, 64, 35, 0.3, 0.6)]
+    with Engine(budget=2 << 30) as eng:
+        eng.config(variant=-1, use_graphs=graphs, chunk=8)
+        mid = eng.add(case)
+        eng.step(32)
+        got = eng.read(mid)
+    o = oracle_mod.OracleRun(case)
+    ts = o.run(case.nsteps)
+    ref, rc = o.layer(0), o.layer(1)
+    for f in ("z", "m", "n"):
+        _same(got[f], ref[f], f)
+        _same(got["child_" + f], rc[f], "child " + f)
+    _same(got["zmax"], ref["zmax"], "zmax")
+    _same(got["ts"], ts, "gauges")
+    assert np.array_equal(got["arrival"], ref["arrival"])
