@@ -1095,12 +1095,11 @@ __device__ __forceinline__ void conmass(const GcLayerDev &L, const float *row, f
  *
  * SPLIT gives the x and y face of a cell to two threads: a small grid leaves
  * most of the chip idle, and the chain of one cell is what it waits for.  The
- * line is at two blocks per SM, where every block is resident in both forms;
- * split against unsplit, when a face still cost 1.4 times as much: 108 blocks
- * 8.1 against 10.8 us, 1197 blocks 21.2 against 21.2, 1748 blocks 28.4
- * against 26.1. */
+ * line is at four blocks per SM; split against unsplit: 320 blocks 9.4
+ * against 10.3 us, 1197 blocks 18.0 against 17.4, 1748 blocks 21.7 against
+ * 21.4. */
 static constexpr int NL_TY = 8;         /* rows of cells per block */
-static constexpr size_t NL_SPLIT = 296; /* blocks up to which SPLIT is taken */
+static constexpr size_t NL_SPLIT = 592; /* blocks up to which SPLIT is taken */
 template <bool SPH, bool ROOT, bool SPLIT>
 __global__ void __launch_bounds__((SPLIT ? 2 : 1) * BX * NL_TY) k_nonlinear_step(GcLayerDev Pl, GcLayerDev L, EdgeArgs E,
                                                                             int upd, int maxamp) {

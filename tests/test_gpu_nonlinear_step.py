@@ -27,7 +27,7 @@ def _same(a, b, what):
 
 
 # child size = cells * ratio + 1
-CHILD = [(2, 2, 3), (10, 2, 3), (9, 5, 7), (21, 13, 3), (13, 3, 5), (33, 9, 7), (80, 29, 7), (84, 33, 7)]
+CHILD = [(2, 2, 3), (10, 2, 3), (9, 5, 7), (21, 13, 3), (13, 3, 5), (33, 9, 7), (80, 29, 7), (84, 33, 7), (110, 37, 7), (117, 38, 7)]
 
 
 @pytest.mark.parametrize("cw,ch,r", CHILD)
