@@ -52,8 +52,11 @@ struct Staging {
         return GC_OK;
     }
     int mark(int k, cudaStream_t s) {
-        GC_CUDA_OR_RET(cudaEventCreateWithFlags(&busy[k], cudaEventDisableTiming));
-        GC_CUDA_OR_RET(cudaEventRecord(busy[k], s));
+        cudaError_t e = cudaEventCreateWithFlags(&busy[k], cudaEventDisableTiming);
+        if (e != cudaSuccess) busy[k] = nullptr;
+        else e = cudaEventRecord(busy[k], s);
+        if (e != cudaSuccess) cudaStreamSynchronize(s); /* nobody else may find the slot in use */
+        GC_CUDA_OR_RET(e);
         return GC_OK;
     }
 };
