@@ -92,16 +92,17 @@ def profiled_traffic(name="fused_linear_step_c2.txt", key="traffic_bytes_per_lau
     return None
 
 
-def pair_note(rl, one_step_gbs, profile):
-    """a two-step launch reads and writes each cell once for two steps, so its
-    HBM fraction is of half the one-step bytes; it is bounded by instruction
-    issue instead.  Adds the HBM fraction a one-step kernel would need for
-    the same steps/s, and the limiter."""
-    if rl.get("steps_per_launch") == 2:
+def pair_note(rl, one_step_gbs):
+    """a launch of several steps reads and writes each cell once for all of
+    them, so its HBM fraction is of a part of the one-step bytes; it is bounded
+    by the arithmetic pipes and instruction issue instead.  Adds the HBM
+    fraction a one-step kernel would need for the same steps/s, and the
+    limiter."""
+    if rl.get("steps_per_launch") > 1:
         rl["one_step_equivalent_gbs"] = one_step_gbs
         rl["one_step_equivalent_frac"] = one_step_gbs / rl["peak"]
-        rl["limiter"] = (f"instruction issue (two steps per HBM pass: same bytes per launch as one step); "
-                         f"issue-slot and stall figures in profiles/{profile}")
+        rl["limiter"] = ("FMA pipe and instruction issue (several steps per HBM pass: same bytes per launch as one "
+                         "step); figures in the kernel's summary under profiles/")
     return rl
 
 
@@ -275,12 +276,30 @@ def timed_engine_steps(torch, eng, steps, warmup, dist, local):
     return ms, launches, ck
 
 
-def steps_per_launch(variant):
-    """2 when the engine's chosen candidate is the two-step kernel
-    (candidates past the one-step variants x their tile-height rules)"""
+BLOCK_FORMS = 8  # the last candidates: the register-tile kernel's forms
+
+
+def steps_per_launch(variant, steps, launches):
+    """steps per launch of the timed window: 1 for the one-step kernel's
+    candidates, 2 for the two-step kernel's after them, and as counted for the
+    register-tile kernel's, whose launches take up to 4 or 8"""
     from comcot_b200 import _lib
 
-    return 2 if variant >= 2 * _lib.load().gc_engine_num_variants() else 1
+    lib = _lib.load()
+    if variant >= lib.gc_engine_num_candidates() - BLOCK_FORMS:
+        return steps / max(1, launches)
+    return 2 if variant >= 2 * lib.gc_engine_num_variants() else 1
+
+
+def profile_name(kind, variant):
+    """the committed counter summary of the candidate's kernel"""
+    from comcot_b200 import _lib
+
+    lib = _lib.load()
+    step = {"linear": "linear_step_c2.txt", "ensemble": "ensemble_step_c4.txt"}[kind]
+    if variant >= lib.gc_engine_num_candidates() - BLOCK_FORMS:
+        return "block_" + step
+    return ("pair_" if variant >= 2 * lib.gc_engine_num_variants() else "fused_") + step
 
 
 def merge_parity(records):
@@ -427,11 +446,10 @@ def bench_c4(torch, dist, world, local, steps, warmup, nscen, plain_sample, vari
             recs.append(parity_record(plain_state, st[steps]["layers"][0], steps, H=L.H,
                                       what="plain path scenario 0 (reference ABI, per phase)"))
     peak, peak_kind = peaks()
-    spl = steps_per_launch(chosen)
+    spl = steps_per_launch(chosen, steps, launches)
     bpc = 24.0 + 4.0 / nscen + 8.0  # per member-cell and launch: Z,M,N in/out, shared H, max-eta r/w
     achieved = bpc * cells * nscen / (ms * 1e-3 / steps * spl) / 1e9
-    tr = profiled_traffic("pair_ensemble_step_c4.txt" if spl == 2 else "fused_ensemble_step_c4.txt",
-                          "traffic_bytes_per_member_launch")
+    tr = profiled_traffic(profile_name("ensemble", chosen), "traffic_bytes_per_member_launch")
     rec = {"metric": "ensemble scenarios/hour", "value": scen_per_hour, "unit": "scenarios/hour",
            "steps": steps, "warmup": warmup, "ms_per_step": ms / steps, "cell_updates_per_s": value_cells,
            "config": {"workload": f"C4: {nscen} dipole scenarios on 1201x1001 2' linear spherical, shared H, "
@@ -442,7 +460,7 @@ def bench_c4(torch, dist, world, local, steps, warmup, nscen, plain_sample, vari
                                   "frac": achieved / peak, "traffic": None if tr is None else nscen * tr,
                                   "peak_kind": f"{peak_kind} (copy bandwidth)",
                                   "algorithmic_bytes_per_launch": bpc * cells * nscen, "steps_per_launch": spl},
-                                 achieved * spl, "pair_ensemble_step_c4.txt"),
+                                 achieved * spl),
            "clocks": ck, "gpu_launches": launches, "parity": merge_parity(recs)}
     if plain:
         rec["plain_path"] = plain
@@ -735,9 +753,11 @@ def run_single(args, torch, dist, rank, world, local):
     tune_reps = 3
     lib = _lib.load()
     ncand = lib.gc_engine_num_candidates()  # the autotuner's candidates: tile variants x tile-height rules
-    # two-step candidates run pairs; the second round re-times the three
-    # fastest over three 64-step graph chunks each
-    total = ncand * (2 * tune_reps + 2) + 3 * 3 * 64 + args.warmup + args.steps + 8
+    # candidates of several steps a launch run whole launches (8 steps at most);
+    # the second round re-times the three fastest over three 64-step graph
+    # chunks each
+    total = (ncand - BLOCK_FORMS) * (2 * tune_reps + 2) + BLOCK_FORMS * 8 * (tune_reps + 1) + 3 * 3 * 64 \
+        + args.warmup + args.steps + 8
     make_case = synth.config_c1 if args.workload == "c1" else synth.config_c2
     case = make_case(nsteps=total)
     cells = case.root.nx * case.root.ny
@@ -793,10 +813,10 @@ def run_single(args, torch, dist, rank, world, local):
         s.close()
 
     peak, peak_kind = peaks()
-    spl = steps_per_launch(variant)
-    bytes_launch = BYTES_PER_CELL * cells  # per launch: one step, or two in the two-step kernel
+    spl = steps_per_launch(variant, args.steps, launches)
+    bytes_launch = BYTES_PER_CELL * cells  # per launch, of however many steps
     achieved = bytes_launch / (ms * 1e-3 / args.steps * spl) / 1e9
-    traffic = profiled_traffic("pair_linear_step_c2.txt" if spl == 2 else "fused_linear_step_c2.txt")
+    traffic = profiled_traffic(profile_name("linear", variant))
     line = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -810,7 +830,7 @@ def run_single(args, torch, dist, rank, world, local):
                                "frac": achieved / peak, "traffic": traffic,
                                "peak_kind": f"{peak_kind} (copy bandwidth)",
                                "algorithmic_bytes_per_launch": bytes_launch, "steps_per_launch": spl},
-                              achieved * spl, "pair_linear_step_c2.txt"),
+                              achieved * spl),
         "clocks": ck,
         "gpu_launches": launches,
     }
