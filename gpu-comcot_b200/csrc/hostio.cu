@@ -67,6 +67,16 @@ bool capturing(cudaStream_t s) {
     return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
 }
 
+/* ordinary host memory: an asynchronous copy from it has read it when the call
+ * returns, while one from page-locked or managed memory reads it when the
+ * stream gets there */
+bool pageable(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
+
 } // namespace
 
 void gc_copy(void *dst, const void *src, size_t bytes) {
@@ -101,6 +111,7 @@ int gc_field_upload(float *d, size_t pitch_bytes, const float *h, int nx, int ny
     const bool staged = total >= kSmall && row <= kSlot && !capturing(s) && (lock.lock(), g_staging.ready());
     if (!staged) {
         GC_CUDA_OR_RET(cudaMemcpy2DAsync(d, pitch_bytes, h, row, row, (size_t)ny, cudaMemcpyHostToDevice, s));
+        if (!pageable(h) && !capturing(s)) GC_CUDA_OR_RET(cudaStreamSynchronize(s));
         return GC_OK;
     }
     const int rows = (int)(kSlot / row);

@@ -7,7 +7,9 @@
 #include "gc_internal.h"
 
 /* nx x ny floats at `h` (contiguous rows) to the pitched device field `d`,
- * in stream order on `s`; the host data has been read when the call returns */
+ * in stream order on `s`; the host data has been read when the call returns,
+ * whatever kind of host memory it is (not on a capturing stream, where the
+ * graph reads page-locked memory at its launch) */
 int gc_field_upload(float *d, size_t pitch_bytes, const float *h, int nx, int ny, cudaStream_t s);
 /* the pitched device field `d` after the work queued on `s`, into `h`; the
  * data is there when the call returns */
