@@ -10,7 +10,13 @@
  *
  * The two buffers (8 MB each) are made at the first transfer of at least
  * 256 KB and kept for the process; a mutex gives them to one call at a time.
- * Where they cannot be had, and for smaller transfers, the plain copy is used.
+ * It is held while a field moves, never while a stream's earlier work runs: a
+ * download, and an upload that fills a buffer twice, first wait for their
+ * stream, and an upload whose stream is busy leaves its copies queued, marks
+ * its buffers and returns.  A call that finds too few buffers free because
+ * another stream's uploads are still queued takes the plain copy, so no caller
+ * waits for another one's steps; so do smaller transfers, and all where the
+ * buffers cannot be had.
  */
 #include <string.h>
 
@@ -30,7 +36,8 @@ struct Staging {
     std::mutex mu;
     bool tried = false;
     char *slot[2] = {nullptr, nullptr};
-    cudaEvent_t busy[2] = {nullptr, nullptr}; /* an upload still reading the slot */
+    cudaEvent_t busy[2] = {nullptr, nullptr}; /* a transfer still using the slot */
+    cudaStream_t by[2] = {nullptr, nullptr};  /* and its stream */
 
     bool ready() {
         if (!tried) {
@@ -42,6 +49,33 @@ struct Staging {
                 }
         }
         return slot[0] && slot[1];
+    }
+    /* Locks the slots for a transfer on `s` that needs `need` of them at once
+     * and gives the first to use; -1, unlocked, where the plain copy is to be
+     * taken.  Slots that earlier uploads on `s` still hold are waited for
+     * outside the lock. */
+    int take(std::unique_lock<std::mutex> &lock, int need, cudaStream_t s) {
+        for (int attempt = 0; attempt < 2; attempt++) {
+            lock.lock();
+            if (!ready()) break;
+            int nfree = 0, first = 0;
+            bool own = false;
+            for (int k = 1; k >= 0; k--) {
+                if (busy[k] && cudaEventQuery(busy[k]) == cudaErrorNotReady) {
+                    cudaGetLastError(); /* an answer, not an error */
+                    own = own || by[k] == s;
+                    continue;
+                }
+                nfree++;
+                first = k;
+            }
+            if (nfree >= need) return first;
+            if (!own) break;
+            lock.unlock();
+            if (cudaStreamSynchronize(s) != cudaSuccess) return -1; /* the plain copy meets the same error */
+        }
+        if (lock.owns_lock()) lock.unlock();
+        return -1;
     }
     int wait(int k) {
         if (!busy[k]) return GC_OK;
@@ -55,6 +89,7 @@ struct Staging {
         cudaError_t e = cudaEventCreateWithFlags(&busy[k], cudaEventDisableTiming);
         if (e != cudaSuccess) busy[k] = nullptr;
         else e = cudaEventRecord(busy[k], s);
+        by[k] = s;
         if (e != cudaSuccess) cudaStreamSynchronize(s); /* nobody else may find the slot in use */
         GC_CUDA_OR_RET(e);
         return GC_OK;
@@ -108,14 +143,20 @@ void gc_copy(void *dst, const void *src, size_t bytes) {
 int gc_field_upload(float *d, size_t pitch_bytes, const float *h, int nx, int ny, cudaStream_t s) {
     const size_t row = (size_t)nx * sizeof(float), total = row * ny;
     std::unique_lock<std::mutex> lock(g_staging.mu, std::defer_lock);
-    const bool staged = total >= kSmall && row <= kSlot && !capturing(s) && (lock.lock(), g_staging.ready());
-    if (!staged) {
+    int first = -1;
+    const bool capture = capturing(s);
+    if (total >= kSmall && row <= kSlot && !capture) {
+        const int rows = (int)(kSlot / row), pieces = (ny + rows - 1) / rows;
+        if (pieces > 2) GC_CUDA_OR_RET(cudaStreamSynchronize(s)); /* the third piece waits for the first copy */
+        first = g_staging.take(lock, std::min(pieces, 2), s);
+    }
+    if (first < 0) {
         GC_CUDA_OR_RET(cudaMemcpy2DAsync(d, pitch_bytes, h, row, row, (size_t)ny, cudaMemcpyHostToDevice, s));
-        if (!pageable(h) && !capturing(s)) GC_CUDA_OR_RET(cudaStreamSynchronize(s));
+        if (!pageable(h) && !capture) GC_CUDA_OR_RET(cudaStreamSynchronize(s));
         return GC_OK;
     }
     const int rows = (int)(kSlot / row);
-    for (int j = 0, k = 0; j < ny; j += rows, k ^= 1) {
+    for (int j = 0, k = first; j < ny; j += rows, k ^= 1) {
         const int n = std::min(rows, ny - j);
         int rc = g_staging.wait(k);
         if (rc != GC_OK) return rc;
@@ -131,8 +172,12 @@ int gc_field_upload(float *d, size_t pitch_bytes, const float *h, int nx, int ny
 int gc_field_download(void *h, const void *d, size_t pitch_bytes, int nx, int ny, cudaStream_t s) {
     const size_t row = (size_t)nx * sizeof(float), total = row * ny;
     std::unique_lock<std::mutex> lock(g_staging.mu, std::defer_lock);
-    const bool staged = total >= kSmall && row <= kSlot && !capturing(s) && (lock.lock(), g_staging.ready());
-    if (!staged) {
+    int first = -1;
+    if (total >= kSmall && row <= kSlot && !capturing(s)) {
+        GC_CUDA_OR_RET(cudaStreamSynchronize(s));
+        first = g_staging.take(lock, 2, s);
+    }
+    if (first < 0) {
         GC_CUDA_OR_RET(cudaMemcpy2DAsync(h, row, d, pitch_bytes, row, (size_t)ny, cudaMemcpyDeviceToHost, s));
         GC_CUDA_OR_RET(cudaStreamSynchronize(s));
         return GC_OK;

@@ -3,6 +3,7 @@
 #include "hostio.cu"
 
 #include <stdio.h>
+#include <unistd.h>
 
 #include <string>
 
@@ -48,6 +49,44 @@ int source(int nx, int ny, cudaMemoryType kind) {
     return 0;
 }
 
+/* a field there and back on a stream of its own */
+int round_trip(FakeStream &s, int nx, int ny) {
+    Field f(nx, ny, 3.0f);
+    std::vector<float> back(f.host.size());
+    CHECK(gc_field_upload(f.dev, f.row(), f.host.data(), nx, ny, &s) == GC_OK);
+    CHECK(gc_field_download(back.data(), f.dev, f.row(), nx, ny, &s) == GC_OK);
+    CHECK(back == f.host && f.there(f.host.data()));
+    return 0;
+}
+
+/* transfers on stream B end while those on stream A wait for A's earlier work:
+ * `uploads` of them queued, then a blocking one (a download, or an upload that
+ * needs its buffers again) in a thread */
+int beside(int nx, int ny, int uploads, bool down) {
+    FakeStream a, b;
+    a.open = false;
+    std::vector<Field> q;
+    q.reserve(uploads + 1);
+    for (int k = 0; k <= uploads; k++) q.emplace_back(nx, ny, 10.0f * k);
+    std::vector<float> back(q[0].host.size());
+    fake::push(&a, [] {}); /* the earlier work */
+    for (int k = 0; k < uploads; k++)
+        CHECK(gc_field_upload(q[k].dev, q[k].row(), q[k].host.data(), nx, ny, &a) == GC_OK);
+    int rc = GC_OK;
+    std::thread t([&] {
+        rc = down ? gc_field_download(back.data(), q[0].dev, q[0].row(), nx, ny, &a)
+                  : gc_field_upload(q[uploads].dev, q[uploads].row(), q[uploads].host.data(), nx, ny, &a);
+    });
+    usleep(200000); /* the thread is waiting by now; were it not, the check would only be weaker */
+    const int mine = round_trip(b, nx, ny) || round_trip(b, 300, 300);
+    fake::set_open(&a, true);
+    t.join();
+    CHECK(mine == 0 && rc == GC_OK && cudaStreamSynchronize(&a) == cudaSuccess);
+    for (int k = 0; k < (down ? uploads : uploads + 1); k++) CHECK(q[k].there(q[k].host.data()));
+    CHECK(!down || uploads == 0 || back == q[0].host);
+    return 0;
+}
+
 } // namespace
 
 int main(int argc, char **argv) {
@@ -56,6 +95,10 @@ int main(int argc, char **argv) {
     if (what == "pageable") return source(nx, ny, cudaMemoryTypeUnregistered);
     if (what == "locked") return source(nx, ny, cudaMemoryTypeHost);
     if (what == "managed") return source(nx, ny, cudaMemoryTypeManaged);
+    alarm(20); /* a transfer that waits for another stream's work would wait for good */
+    if (what == "beside-read") return beside(nx, ny, 0, true);
+    if (what == "beside-queued-read") return beside(nx, ny, 1, true);
+    if (what == "beside-upload") return beside(nx, ny, 2, false);
     printf("no scenario %s\n", what.c_str());
     return 2;
 }

@@ -29,3 +29,9 @@ def scenario(tmp_path_factory):
 @pytest.mark.parametrize("kind", ["pageable", "locked", "managed"])
 def test_source_may_change_after_an_upload(scenario, kind, nx, ny):
     scenario(kind, nx, ny)
+
+
+@pytest.mark.parametrize("nx,ny", [(300, 300), (1201, 1001), (2401, 801)])   # a quarter of a slot, one slot, nearly one
+@pytest.mark.parametrize("kind", ["beside-read", "beside-queued-read", "beside-upload"])
+def test_transfers_do_not_wait_for_another_streams_work(scenario, kind, nx, ny):
+    scenario(kind, nx, ny)
