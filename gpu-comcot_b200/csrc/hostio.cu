@@ -85,8 +85,19 @@ struct Staging {
         GC_CUDA_OR_RET(e);
         return GC_OK;
     }
+    /* the event belongs to the stream's device, whichever is current */
+    static cudaError_t make_event(cudaEvent_t *ev, cudaStream_t s) {
+        int dev = 0, cur = 0;
+        cudaError_t e = cudaGetDevice(&cur);
+        if (e == cudaSuccess) e = cudaStreamGetDevice(s, &dev);
+        if (e == cudaSuccess && dev != cur) e = cudaSetDevice(dev);
+        if (e != cudaSuccess) return e;
+        e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        if (dev != cur) cudaSetDevice(cur);
+        return e;
+    }
     int mark(int k, cudaStream_t s) {
-        cudaError_t e = cudaEventCreateWithFlags(&busy[k], cudaEventDisableTiming);
+        cudaError_t e = make_event(&busy[k], s);
         if (e != cudaSuccess) busy[k] = nullptr;
         else e = cudaEventRecord(busy[k], s);
         by[k] = s;

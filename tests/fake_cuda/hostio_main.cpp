@@ -87,6 +87,15 @@ int beside(int nx, int ny, int uploads, bool down) {
     return 0;
 }
 
+/* a thread whose current device is not the stream's */
+int foreign(int nx, int ny) {
+    FakeStream s;
+    s.device = 1;
+    CHECK(round_trip(s, nx, ny) == 0);
+    CHECK(fake::device == 0);
+    return 0;
+}
+
 } // namespace
 
 int main(int argc, char **argv) {
@@ -99,6 +108,7 @@ int main(int argc, char **argv) {
     if (what == "beside-read") return beside(nx, ny, 0, true);
     if (what == "beside-queued-read") return beside(nx, ny, 1, true);
     if (what == "beside-upload") return beside(nx, ny, 2, false);
+    if (what == "foreign-device") return foreign(nx, ny);
     printf("no scenario %s\n", what.c_str());
     return 2;
 }

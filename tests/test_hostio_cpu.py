@@ -35,3 +35,8 @@ def test_source_may_change_after_an_upload(scenario, kind, nx, ny):
 @pytest.mark.parametrize("kind", ["beside-read", "beside-queued-read", "beside-upload"])
 def test_transfers_do_not_wait_for_another_streams_work(scenario, kind, nx, ny):
     scenario(kind, nx, ny)
+
+
+@pytest.mark.parametrize("nx,ny", [(33, 17), (300, 300), (2401, 2001)])
+def test_transfers_on_a_device_that_is_not_current(scenario, nx, ny):
+    scenario("foreign-device", nx, ny)
