@@ -15,7 +15,8 @@
  * stream, and an upload whose stream is busy leaves its copies queued, marks
  * its buffers and returns.  A call that finds too few buffers free because
  * another stream's uploads are still queued takes the plain copy, so no caller
- * waits for another one's steps; so do smaller transfers, and all where the
+ * waits for another one's steps; so do smaller transfers, those whose caller's
+ * side is device memory, which host threads cannot touch, and all where the
  * buffers cannot be had.
  */
 #include <string.h>
@@ -113,14 +114,14 @@ bool capturing(cudaStream_t s) {
     return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
 }
 
-/* ordinary host memory: an asynchronous copy from it has read it when the call
- * returns, while one from page-locked or managed memory reads it when the
- * stream gets there */
-bool pageable(const void *p) {
+/* Whose memory a caller's pointer names.  An asynchronous copy from ordinary
+ * host memory has read it when the call returns, while one from page-locked,
+ * managed or device memory reads it when the stream gets there. */
+cudaMemoryType memory_of(const void *p) {
     cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type;
     cudaGetLastError();
-    return false;
+    return cudaMemoryTypeHost; /* unknown: waited for */
 }
 
 } // namespace
@@ -156,14 +157,15 @@ int gc_field_upload(float *d, size_t pitch_bytes, const float *h, int nx, int ny
     std::unique_lock<std::mutex> lock(g_staging.mu, std::defer_lock);
     int first = -1;
     const bool capture = capturing(s);
-    if (total >= kSmall && row <= kSlot && !capture) {
+    const cudaMemoryType from = memory_of(h);
+    if (total >= kSmall && row <= kSlot && !capture && from != cudaMemoryTypeDevice) {
         const int rows = (int)(kSlot / row), pieces = (ny + rows - 1) / rows;
         if (pieces > 2) GC_CUDA_OR_RET(cudaStreamSynchronize(s)); /* the third piece waits for the first copy */
         first = g_staging.take(lock, std::min(pieces, 2), s);
     }
     if (first < 0) {
         GC_CUDA_OR_RET(cudaMemcpy2DAsync(d, pitch_bytes, h, row, row, (size_t)ny, cudaMemcpyHostToDevice, s));
-        if (!pageable(h) && !capture) GC_CUDA_OR_RET(cudaStreamSynchronize(s));
+        if (from != cudaMemoryTypeUnregistered && !capture) GC_CUDA_OR_RET(cudaStreamSynchronize(s));
         return GC_OK;
     }
     const int rows = (int)(kSlot / row);
@@ -184,7 +186,7 @@ int gc_field_download(void *h, const void *d, size_t pitch_bytes, int nx, int ny
     const size_t row = (size_t)nx * sizeof(float), total = row * ny;
     std::unique_lock<std::mutex> lock(g_staging.mu, std::defer_lock);
     int first = -1;
-    if (total >= kSmall && row <= kSlot && !capturing(s)) {
+    if (total >= kSmall && row <= kSlot && !capturing(s) && memory_of(h) != cudaMemoryTypeDevice) {
         GC_CUDA_OR_RET(cudaStreamSynchronize(s));
         first = g_staging.take(lock, 2, s);
     }

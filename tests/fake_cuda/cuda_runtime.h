@@ -2,8 +2,8 @@
  * A CUDA runtime of host memory for tests of host code: the calls the field
  * transfers make, on streams that run what is queued on them only when a test
  * or a wait lets them.  "Device" memory is host memory; page-locked memory is
- * what cudaHostAlloc returned, device memory what fake_device returned; every
- * other pointer is pageable.  Copies from or to pageable memory behave as the
+ * what cudaHostAlloc returned, other kinds come from fake::make; every other
+ * pointer is pageable.  Copies from or to pageable memory behave as the
  * runtime documents them: the source has been read, the destination has been
  * written, when the call returns.
  */
@@ -50,6 +50,7 @@ inline std::mutex mu;
 inline std::condition_variable cv;
 inline std::map<const char *, std::pair<size_t, cudaMemoryType>> known; /* start -> size, kind */
 inline thread_local int device = 0;
+inline int device_callers = 0; /* copies whose caller's side is device memory */
 
 inline cudaMemoryType kind(const void *p) {
     auto it = known.upper_bound((const char *)p);
@@ -138,7 +139,7 @@ inline cudaError_t cudaMemcpy2DAsync(void *d, size_t dp, const void *s, size_t s
     std::unique_lock<std::mutex> l(fake::mu);
     const bool up = dir == cudaMemcpyHostToDevice;
     const cudaMemoryType k = fake::kind(up ? s : d);
-    if (k == cudaMemoryTypeDevice) return cudaErrorInvalidValue;
+    fake::device_callers += k == cudaMemoryTypeDevice;
     if (k != cudaMemoryTypeUnregistered) {
         fake::push(st, [=] { rows((char *)d, dp, (const char *)s, sp); });
     } else if (up) {

@@ -96,6 +96,18 @@ int foreign(int nx, int ny) {
     return 0;
 }
 
+/* device memory on the caller's side: the runtime's own copies, no host access */
+int device_caller(int nx, int ny) {
+    CHECK(source(nx, ny, cudaMemoryTypeDevice) == 0 && fake::device_callers == 1);
+    FakeStream s;
+    Field f(nx, ny, 2.0f);
+    float *to = (float *)fake::make(f.host.size() * sizeof(float), cudaMemoryTypeDevice);
+    CHECK(gc_field_upload(f.dev, f.row(), f.host.data(), nx, ny, &s) == GC_OK);
+    CHECK(gc_field_download(to, f.dev, f.row(), nx, ny, &s) == GC_OK && fake::device_callers == 2);
+    CHECK(memcmp(to, f.host.data(), f.host.size() * sizeof(float)) == 0);
+    return 0;
+}
+
 } // namespace
 
 int main(int argc, char **argv) {
@@ -109,6 +121,7 @@ int main(int argc, char **argv) {
     if (what == "beside-queued-read") return beside(nx, ny, 1, true);
     if (what == "beside-upload") return beside(nx, ny, 2, false);
     if (what == "foreign-device") return foreign(nx, ny);
+    if (what == "device-caller") return device_caller(nx, ny);
     printf("no scenario %s\n", what.c_str());
     return 2;
 }

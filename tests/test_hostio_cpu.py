@@ -40,3 +40,8 @@ def test_transfers_do_not_wait_for_another_streams_work(scenario, kind, nx, ny):
 @pytest.mark.parametrize("nx,ny", [(33, 17), (300, 300), (2401, 2001)])
 def test_transfers_on_a_device_that_is_not_current(scenario, nx, ny):
     scenario("foreign-device", nx, ny)
+
+
+@pytest.mark.parametrize("nx,ny", [(33, 17), (300, 300), (2401, 2001)])
+def test_callers_device_memory_is_left_to_the_runtime(scenario, nx, ny):
+    scenario("device-caller", nx, ny)
