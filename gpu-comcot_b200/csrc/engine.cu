@@ -1304,6 +1304,7 @@ int gc_engine_config(gc_engine *e, int variant, int use_graphs, int graph_chunk)
  * tuning steps are ordinary steps of the run. */
 int gc_engine_autotune(gc_engine *e, int reps) {
     if (!e || reps < 1) return GC_EINVAL;
+    e->tuned = true; /* the rebuild of each candidate keeps the candidate's form */
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
@@ -1361,7 +1362,6 @@ int gc_engine_autotune(gc_engine *e, int reps) {
     }
     if (best < 0) best = e->pair_allowed ? n1 : 16;
     eng_set_candidate(e, best);
-    e->tuned = true;
     e->use_graphs = saved_graphs;
     e->dirty = true;
     cudaEventDestroy(a);
