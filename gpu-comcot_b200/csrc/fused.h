@@ -78,8 +78,8 @@ cudaError_t gc_fused_launch_multi(int variant, const GcFusedGrid *d_grids, const
 int gc_fused_max_ctas(int variant, bool multi = true);
 /* 1 if a pipeline wait in the fused kernel gave up since the last call (clears it) */
 int gc_fused_take_error();
-/* that flag's device address */
-cudaError_t gc_fused_error_flag(int **flag);
+/* sets that flag from the host, as a wait that gives up sets it */
+int gc_fused_raise_error();
 /* single grid, descriptor by value */
 cudaError_t gc_fused_launch_one(int variant, const GcFusedGrid &g, int step, cudaStream_t s);
 /* single grid at step step_off + *d_step_base (d_step_base may be NULL) */
@@ -171,7 +171,7 @@ cudaError_t gc_block_launch_class(int variant, const GcPairClass &c, int T, cons
 /* ---- one step, warps on their own (kernels_step.cu): factored R2/R4, the
  * outermost layer, no gauges, arrival by max-eta ---- */
 cudaError_t gc_step_launch_one(const GcFusedGrid &g, const int *d_step_base, int step_off, cudaStream_t s);
-/* up to 64 grids by value; clear: a device flag to set to 0, or NULL */
-cudaError_t gc_step_launch_grids(int n, const GcFusedGrid *g, int step, int *clear, cudaStream_t s);
+/* up to 64 grids by value */
+cudaError_t gc_step_launch_grids(int n, const GcFusedGrid *g, int step, cudaStream_t s);
 
 #endif

@@ -668,7 +668,10 @@ int gc_fused_take_error() {
     return v;
 }
 
-cudaError_t gc_fused_error_flag(int **flag) { return cudaGetSymbolAddress((void **)flag, g_pipe_error); }
+int gc_fused_raise_error() {
+    const int one = 1;
+    return cudaMemcpyToSymbol(g_pipe_error, &one, sizeof one) == cudaSuccess ? GC_OK : GC_ECUDA;
+}
 
 GcTileCfg gc_fused_variant(int v) {
     if (v < 0 || v >= kNumVariants) v = 0;

@@ -275,14 +275,12 @@ __global__ void __launch_bounds__(32 * SWARPS) k_step_one(const __grid_constant_
 template <int N>
 struct StepGrids {
     int n, start[N + 1], tx[N];
-    int *clear; /* a flag to set to 0 in stream order, or NULL */
     GcFusedGrid g[N];
 };
 static_assert(sizeof(StepGrids<64>) <= 32000, "kernel parameters may take up to 32764 bytes");
 template <int R, int N>
 __global__ void __launch_bounds__(32 * SWARPS) k_step_grids(const __grid_constant__ StepGrids<N> p, int step) {
     pdl_enter();
-    if (p.clear && blockIdx.x == 0 && threadIdx.x == 0) *p.clear = 0;
     int lo = 0, hi = p.n - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -315,13 +313,12 @@ cudaError_t launch_step(void (*kern)(K...), long long ctas, cudaStream_t s, cons
 int step_rows_for(long long cells) { return cells < 2000000 ? 1 : 2; }
 
 template <int N>
-cudaError_t launch_grids(int n, const GcFusedGrid *g, int step, int *clear, cudaStream_t s) {
+cudaError_t launch_grids(int n, const GcFusedGrid *g, int step, cudaStream_t s) {
     StepGrids<N> p; /* on this thread's stack: the launch copies it */
     long long cells = 0;
     for (int k = 0; k < n; k++) cells += (long long)g[k].nx * g[k].ny;
     const int R = step_rows_for(cells);
     p.n = n;
-    p.clear = clear;
     long long t = 0;
     for (int k = 0; k < n; k++) {
         p.g[k] = g[k];
@@ -344,7 +341,7 @@ cudaError_t gc_step_launch_one(const GcFusedGrid &g, const int *d_step_base, int
                   : launch_step(k_step_one<2>, ctas, s, g, d_step_base, step_off, ntx);
 }
 
-cudaError_t gc_step_launch_grids(int n, const GcFusedGrid *g, int step, int *clear, cudaStream_t s) {
+cudaError_t gc_step_launch_grids(int n, const GcFusedGrid *g, int step, cudaStream_t s) {
     if (n < 1 || n > 64) return cudaErrorInvalidValue;
-    return n <= 4 ? launch_grids<4>(n, g, step, clear, s) : launch_grids<64>(n, g, step, clear, s);
+    return n <= 4 ? launch_grids<4>(n, g, step, s) : launch_grids<64>(n, g, step, s);
 }

@@ -19,11 +19,10 @@
  * one-warp-per-tile step: three launches a call, and a 361 x 301 grid's 87
  * tiles kept 29 CTAs of 148 SMs busy for 20 us.
  *
- * The first call on each device looks up the library's error flag; make it
- * before any stream capture.  Each call clears that flag in stream order, and
- * gcomcot_sync() reads it.
+ * The kernel has no waits, so it neither raises nor clears the flag that
+ * gcomcot_sync() reports, and no call sets anything up: the first one may be
+ * made inside a stream capture.
  */
-#include <mutex>
 #include <string.h>
 
 #include "fused.h"
@@ -33,10 +32,6 @@
 #define GC_NOALLOC_MAX_TILES 24576
 
 namespace {
-
-constexpr int kMaxDevices = 64;
-int *g_flag[kMaxDevices] = {nullptr}; /* the error flag's address per device */
-std::mutex g_mu;
 
 bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
@@ -89,22 +84,6 @@ extern "C" int gcomcot_fused_step_noalloc(int ngrids, const gc_grid_step_io *gri
         d.n[0] = const_cast<float *>(q.n1); d.n[1] = q.n2;
         d.h = q.h; d.rows = q.rows; d.zmax = q.zmax;
     }
-    int *flag = nullptr;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        int dev = 0;
-        GC_CUDA_OR_RET(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= kMaxDevices) return GC_ENOTSUP;
-        if (!g_flag[dev]) {
-            /* once per device, with that device current */
-            cudaError_t e = gc_fused_error_flag(&g_flag[dev]);
-            if (e != cudaSuccess || !g_flag[dev]) {
-                fprintf(stderr, "gcomcot_fused_step_noalloc: cudaGetSymbolAddress: %s\n", cudaGetErrorString(e));
-                return GC_ECUDA;
-            }
-        }
-        flag = g_flag[dev];
-    }
-    GC_CUDA_OR_RET(gc_step_launch_grids(ngrids, desc, 1, flag, (cudaStream_t)stream));
+    GC_CUDA_OR_RET(gc_step_launch_grids(ngrids, desc, 1, (cudaStream_t)stream));
     return GC_OK;
 }

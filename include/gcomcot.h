@@ -118,6 +118,9 @@ void gcomcot_set_wait_limit(int polls);
  * issued for it), so the bounded wait above gives up; for tests of the
  * failure path without faulting a GPU */
 void gcomcot_inject_stall(void);
+/* diagnostics: sets the error flag of the one-step kernel from the host, as a
+ * bounded wait of a launch that gave up would have; 0 or a negative status */
+int gcomcot_inject_timeout(void);
 
 /* Runs `nsteps` outer steps through the Part-1 entry points in the order of
  * comcot.f90:359-439 (MASS, OPEN, ALL_GRID, MOMENT, MAX_AMP, GET_TS per
@@ -296,9 +299,8 @@ typedef struct {
  * one launch on `stream` (at most 64 grids, and 24576 tiles of 128 columns by
  * 4096 rows; larger requests return -1).  The grid list travels in the launch
  * parameters, so nothing is copied from host memory, the library holds no
- * device memory for it, and the call returns once its launch is queued.  The
- * first call on a device does a one-time set-up and should come before any
- * stream capture.  Returns 0 or a negative status. */
+ * device memory for it, and the call returns once its launch is queued.
+ * Returns 0 or a negative status. */
 int gcomcot_fused_step_noalloc(int ngrids, const gc_grid_step_io *grids, void *stream);
 
 #ifdef __cplusplus
