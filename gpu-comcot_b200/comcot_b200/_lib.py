@@ -82,6 +82,7 @@ SIGNATURES = {
     "gcomcot_set_wait_limit": (None, [C.c_int]),
     "gcomcot_inject_stall": (None, []),
     "gcomcot_inject_timeout": (C.c_int, []),
+    "gcomcot_set_block_limit": (None, [C.c_longlong]),
     "gcomcot_drive": (C.c_int, [C.c_int, C.c_int, C.c_int, P_I, P_I, P_I, P_F]),
     "gc_engine_create": (C.c_int, [C.c_longlong, C.POINTER(VP)]),
     "gc_engine_destroy": (C.c_int, [VP]),

@@ -112,6 +112,8 @@ void gcomcot_set_wait_limit(int polls) { gc_pair_set_wait_limit(polls); }
 
 void gcomcot_inject_stall(void) { gc_pair_stall_next(); }
 
+void gcomcot_set_block_limit(long long bytes) { gc_block_set_field_limit(bytes); }
+
 int gcomcot_inject_timeout(void) { return gc_fused_raise_error(); }
 
 /* the library's stream, for callers that time work with CUDA events */

@@ -198,26 +198,35 @@ int gcomcot_drive(int nsteps, int maxamp, int ngauges, const int *g_layer, const
     };
     int k = 0;
     if (nsteps >= 1 && drive_block_ok(R, maxamp, ngauges, g_layer)) {
-        /* each launch (kernels_block.cu) reads the current level (buffer A)
-         * and writes the level t steps on into the other buffer (B); the levels
+        /* each launch (kernels_block.cu; where the grid does not fit it, two
+         * steps of kernels_pair.cu) reads the current level (buffer A) and
+         * writes the level t steps on into the other buffer (B); the levels
          * between are never stored.  Their gauge stencils are recorded inside
          * the launch.  The last step's are taken by the next launch as it
          * starts (from the level it reads), or by the gauge kernel when no
          * launch of the same history chunk follows. */
+        constexpr int kPairVariant = 7; /* 1 warp x 5 stages, the fastest single-grid form on B200 */
         int variant = 0, most = 1;
         gc_block_form(gc_block_pick_form(1, &R.nx, &R.ny), &variant, &most);
         GcFusedGrid g;
         gc_fill_fused_grid(R, g);
         gc_block_plan(variant, g, most);
-        const bool fits = gc_block_fits(g, 1); /* else one step at a time below */
+        const bool block = gc_block_fits(g, 1);
+        if (!block) {
+            most = 2;
+            g.pty = gc_pair_pick_ty(kPairVariant, 1, &R.nx, &R.ny, 2, false);
+            g.pte = gc_pair_short_ty(2, g.pty);
+            gc_pair_tiles(R.nx, R.ny, g.pty, g.pte, &g.ptiles_x);
+        }
+        const int least = block ? 1 : 2; /* a last step alone is left to the loop below */
         g.nbuf = 3;
         g.step0 = 0;
-        g.nsteps = most + 2;
+        g.nsteps = most + 1 + (block ? 1 : 0);
         g.flags = GC_F_MAXAMP | (ngauges > 0 ? GC_F_STENCIL : 0);
         g.ng = ngauges;
         g.gij = d_ij;
         g.gw = nullptr;
-        while (fits && k < nsteps && rc == GC_OK) {
+        while (nsteps - k >= least && rc == GC_OK) {
             const int A = R.cur, B = A ^ 1;
             /* local step 1 when the previous step's slot is in this history
              * chunk: the launch then also samples the level it reads into that
@@ -225,7 +234,7 @@ int gcomcot_drive(int nsteps, int maxamp, int ngauges, const int *g_layer, const
              * buffer L % 3, so t is not a multiple of 3. */
             const int local = (ngauges > 0 && k % chunk > 0) ? 1 : 0;
             int t = std::min(most, nsteps - k);
-            if (ngauges > 0) t = std::min(t, chunk - k % chunk);
+            if (ngauges > 0) t = std::min(t, chunk - k % chunk); /* the chunk is even: so are pairs */
             if (t % 3 == 0) t--;
             for (int q = 0; q < 3; q++) { /* the buffer read is level `local`'s, every other one names B */
                 g.z[q] = R.z[q == local ? A : B]; g.m[q] = R.m[q == local ? A : B];
@@ -234,14 +243,16 @@ int gcomcot_drive(int nsteps, int maxamp, int ngauges, const int *g_layer, const
             g.ts = ngauges > 0 ? d_hist + (size_t)(k % chunk - local) * ngauges * 4 : nullptr;
             {
                 GcPdlScope pdl(true);
-                if (gc_block_launch_one(variant, g, t, nullptr, local, rt.stream) != cudaSuccess) rc = GC_ECUDA;
+                const cudaError_t e = block ? gc_block_launch_one(variant, g, t, nullptr, local, rt.stream)
+                                            : gc_pair_launch_one_at(kPairVariant, g, nullptr, local, rt.stream);
+                if (e != cudaSuccess) rc = GC_ECUDA;
             }
             rt.launches++;
             k += t;
             if (ngauges > 0) {
                 /* the next launch samples this one's last step when it exists
                  * and that step's slot is not the last of its chunk */
-                const bool next_samples = k < nsteps && k % chunk != 0;
+                const bool next_samples = nsteps - k >= least && k % chunk != 0;
                 if (!next_samples) gauges_after(k - 1, R.z[B]);
                 flush_hist(k - 1);
             }

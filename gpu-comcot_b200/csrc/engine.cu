@@ -190,6 +190,7 @@ struct gc_engine {
     GcPairClass pcls;
     /* several steps per launch, tiles in registers (kernels_block.cu) */
     int block_on = 1;             /* the chosen candidate uses it */
+    bool block_now = true;        /* and every active member's windows fit it */
     int block_form = 0, block_variant = 0, block_T = 4;
     int2 *d_btiles = nullptr;
     int btiles_cap = 0, nbtiles = 0;
@@ -423,7 +424,7 @@ static cudaError_t eng_launch_steps_(gc_engine *e, const int *d_base, int step_o
         /* two steps per launch while both lie inside every member's window
          * (the launch after a member's last step only samples its gauges) */
         int k = 0;
-        if (e->block_on && e->pair_ok)
+        if (e->block_now && e->pair_ok)
             while (k < count) {
                 /* the most steps the margin, the request and the members'
                  * windows allow; a launch must not write the buffer it reads
@@ -439,7 +440,7 @@ static cudaError_t eng_launch_steps_(gc_engine *e, const int *d_base, int step_o
                 e->launches++;
                 k += t;
             }
-        if (e->pair_ok && !e->block_on)
+        if (e->pair_ok && !e->block_now)
             for (; k + 1 < count && k + 2 <= pair_room; k += 2) {
                 cudaError_t err = e->single
                                       ? gc_pair_launch_one_at(e->pair_variant, e->one_grid, d_base, step_off0 + k,
@@ -490,6 +491,23 @@ static int eng_make_aux(gc_engine *e, int naux) {
     return GC_OK;
 }
 
+/* whether the register-tile form in force can step every active member; else
+ * the members go two steps at a time through kernels_pair.cu, whose offsets are
+ * 64 bits wide */
+static bool eng_block_fits(const gc_engine *e) {
+    for (size_t c = 0; c < e->classes.size(); c++) {
+        int n = 0;
+        for (const EngMember &M : e->members) n += M.used && !M.done && !M.nested && M.cls == (int)c;
+        if (n == 0) continue;
+        GcFusedGrid g;
+        memset(&g, 0, sizeof g);
+        g.nx = e->classes[c].nx; g.ny = e->classes[c].ny; g.pitch = e->classes[c].pitch;
+        gc_block_plan(e->block_variant, g, e->block_T);
+        if (!gc_block_fits(g, n)) return false;
+    }
+    return true;
+}
+
 static int eng_rebuild(gc_engine *e) {
     std::vector<GcFusedGrid> grids;
     std::vector<int2> tiles;
@@ -509,6 +527,7 @@ static int eng_rebuild(gc_engine *e) {
         e->block_form = gc_block_pick_form((int)anx.size(), anx.data(), any.data());
         gc_block_form(e->block_form, &e->block_variant, &e->block_T);
     }
+    e->block_now = e->block_on && eng_block_fits(e);
     const int ty = anx.empty() ? 16 : gc_fused_pick_ty(e->variant, (int)anx.size(), anx.data(), any.data(),
                                                        e->ty_rule, !single);
     const int pty = anx.empty() ? 32 : gc_pair_pick_ty(e->pair_variant, (int)anx.size(), anx.data(), any.data(),
@@ -517,7 +536,6 @@ static int eng_rebuild(gc_engine *e) {
     /* two-step launches need at most 64 gauges per member */
     bool pair_ok = (e->pair_on != 0 || e->block_on != 0) && e->pair_allowed != 0 && !anx.empty();
     std::vector<int2> ptiles, btiles;
-    bool block_fits = true; /* fields beyond 4 GB go through the one-step kernel */
     /* active members grouped by class */
     for (size_t c = 0; c < e->classes.size(); c++) {
         EngClass &C = e->classes[c];
@@ -537,7 +555,7 @@ static int eng_rebuild(gc_engine *e) {
             g.nbuf = 3;
             g.pty = pty;
             g.pte = pte;
-            if (e->block_on) gc_block_plan(e->block_variant, g, e->block_T);
+            if (e->block_now) gc_block_plan(e->block_variant, g, e->block_T);
             gc_pair_tiles(C.nx, C.ny, pty, pte, &g.ptiles_x);
             for (int q = 0; q < 3; q++) { g.z[q] = M.z[q]; g.m[q] = M.m[q]; g.n[q] = M.n[q]; }
             g.h = M.h ? M.h : C.d_h; g.rows = C.d_rows;
@@ -549,11 +567,10 @@ static int eng_rebuild(gc_engine *e) {
         int nt = gc_fused_tiles(C.nx, C.ny, ty, nullptr);
         for (int t = 0; t < nt; t++)
             for (int g : idx) tiles.push_back(make_int2(g, t));
-        const int npt = e->block_on ? 0 : gc_pair_tiles(C.nx, C.ny, pty, pte, nullptr);
+        const int npt = e->block_now ? 0 : gc_pair_tiles(C.nx, C.ny, pty, pte, nullptr);
         for (int t = 0; t < npt; t++)
             for (int g : idx) ptiles.push_back(make_int2(g, t));
-        if (e->block_on && !gc_block_fits(grids[idx[0]], (int)idx.size())) block_fits = false;
-        if (e->block_on && block_fits) {
+        if (e->block_now) {
             const int nbt = grids[idx[0]].bntx * grids[idx[0]].bnty;
             for (int t = 0; t < nbt; t++)
                 for (int g : idx) btiles.push_back(make_int2(g, t));
@@ -591,7 +608,6 @@ static int eng_rebuild(gc_engine *e) {
     if (e->nptiles)
         GC_CUDA_OR_RET(cudaMemcpyAsync(e->d_ptiles, ptiles.data(), ptiles.size() * sizeof(int2),
                                        cudaMemcpyHostToDevice, e->stream));
-    if (!block_fits) pair_ok = false;
     e->nbtiles = (int)btiles.size();
     if (e->nbtiles > e->btiles_cap) {
         if (e->d_btiles) cudaFreeAsync(e->d_btiles, e->stream);
@@ -683,7 +699,7 @@ static int eng_issue(gc_engine *e, int nsteps) {
         /* the register-tile launches last longer than the host takes to issue
          * one, so without nested chains they go out as they are, and no graph
          * has to be captured when the members change */
-        const bool graphs = e->use_graphs && !(e->block_on && e->pair_ok && e->nested_ids.empty());
+        const bool graphs = e->use_graphs && !(e->block_now && e->pair_ok && e->nested_ids.empty());
         if (graphs && horizon >= e->chunk && (!e->pair_ok || room >= e->chunk)) {
             /* the device counter must equal the host's step count */
             GC_CUDA_OR_RET(cudaMemcpyAsync(e->d_step, &e->gstep, sizeof(int), cudaMemcpyHostToDevice, e->stream));
@@ -1268,6 +1284,7 @@ static bool eng_set_candidate(gc_engine *e, int c) {
     if (c < 0 || c >= eng_num_candidates()) return false;
     const int n2 = n1 + np * GC_PAIR_RULES;
     e->block_on = 0;
+    e->block_now = true;
     if (c >= n2) {
         e->block_form = c - n2;
         gc_block_form(e->block_form, &e->block_variant, &e->block_T);
@@ -1337,6 +1354,7 @@ int gc_engine_autotune(gc_engine *e, int reps) {
     bool short_of_steps = false;
     for (int c = 0; c < eng_num_candidates(); c++) {
         if (c >= n1 && !e->pair_allowed) break;
+        if (eng_set_candidate(e, c) && e->block_on && !eng_block_fits(e)) continue;
         const float ms = time_candidate(c, 1);
         if (ms < 0.0f) {
             short_of_steps = true;
@@ -1374,7 +1392,7 @@ int gc_engine_prepare(gc_engine *e) {
     eng_retire(e);
     if (e->dirty && eng_rebuild(e) != GC_OK) return GC_ECUDA;
     if (e->use_graphs && !e->gexec && (e->ntiles > 0 || !e->nested_ids.empty()) &&
-        !(e->block_on && e->pair_ok && e->nested_ids.empty()))
+        !(e->block_now && e->pair_ok && e->nested_ids.empty()))
         GC_CUDA_OR_RET(eng_build_graph(e));
     GC_CUDA_OR_RET(cudaStreamSynchronize(e->stream));
     return GC_OK;
@@ -1382,7 +1400,7 @@ int gc_engine_prepare(gc_engine *e) {
 
 int gc_engine_variant(gc_engine *e) {
     if (!e) return GC_EINVAL;
-    if (e->block_on && e->pair_allowed)
+    if (e->block_on && e->block_now && e->pair_allowed)
         return gc_fused_num_variants() * GC_TY_RULES + gc_pair_num_variants() * GC_PAIR_RULES + e->block_form;
     if (e->pair_on && e->pair_allowed)
         return gc_fused_num_variants() * GC_TY_RULES + e->pair_variant + gc_pair_num_variants() * e->pair_rule;

@@ -13,7 +13,7 @@
  * max-eta every step and start arrival at 0 where the initial surface is
  * already above the threshold on a wet cell) */
 #define GC_F_ARR_BYMAX 4
-/* register-tile kernel: gauge records are the raw 2x2 surface stencils (four
+/* register-tile and two-step kernels: gauge records are the raw 2x2 surface stencils (four
  * values per gauge and step, as gcomcot_get_z_ returns them) instead of the
  * GET_TS bilinear value */
 #define GC_F_STENCIL 8
@@ -155,6 +155,9 @@ int gc_block_pick_form(int ngrids, const int *nx, const int *ny);
 /* whether a planned grid's byte offsets and window numbers fit 32 bits
  * (`members` of them in a class launch) */
 bool gc_block_fits(const GcFusedGrid &g, int members);
+/* diagnostics: the bytes of a field from which on a grid does not fit (at most
+ * 4 GB, where its offsets run out; <= 0 restores that) */
+void gc_block_set_field_limit(long long bytes);
 /* fills a grid's window layout for launches of up to bt steps; returns the
  * number of windows */
 int gc_block_plan(int variant, GcFusedGrid &g, int bt);

@@ -60,6 +60,9 @@
  */
 #include <math.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "fused.h"
 #include "packed.cuh"
 
@@ -848,9 +851,15 @@ cudaError_t launch_block(void (*kern)(K...), const BlockVariant &v, int ctas, cu
 
 } // namespace
 
+static std::atomic<unsigned long long> g_field_limit{1ull << 32}; /* bytes of a field: its offsets have 32 bits */
+
+void gc_block_set_field_limit(long long bytes) {
+    g_field_limit = bytes > 0 ? std::min((unsigned long long)bytes, 1ull << 32) : 1ull << 32;
+}
+
 bool gc_block_fits(const GcFusedGrid &g, int members) {
     const unsigned long long lim = 1ull << 32, n = (unsigned long long)g.bntx * g.bnty;
-    return 4ull * g.pitch * g.ny < lim && n * g.bntx < lim && n * members * members < lim;
+    return 4ull * g.pitch * g.ny < g_field_limit && n * g.bntx < lim && n * members * members < lim;
 }
 
 /* ceil(2^32 / d): (k * that) >> 32 is k / d while k * d < 2^32 */

@@ -118,6 +118,11 @@ void gcomcot_set_wait_limit(int polls);
  * issued for it), so the bounded wait above gives up; for tests of the
  * failure path without faulting a GPU */
 void gcomcot_inject_stall(void);
+/* diagnostics: the bytes of a field from which on engine members and
+ * gcomcot_drive leave the register-tile kernel for the two-step one (4 GB, where
+ * its 32-bit offsets run out; <= 0 restores that); for tests of that path
+ * without such a grid */
+void gcomcot_set_block_limit(long long bytes);
 /* diagnostics: sets the error flag of the one-step kernel from the host, as a
  * bounded wait of a launch that gave up would have; 0 or a negative status */
 int gcomcot_inject_timeout(void);
