@@ -496,14 +496,14 @@ static int eng_make_aux(gc_engine *e, int naux) {
  * 64 bits wide */
 static bool eng_block_fits(const gc_engine *e) {
     for (size_t c = 0; c < e->classes.size(); c++) {
-        int n = 0;
-        for (const EngMember &M : e->members) n += M.used && !M.done && !M.nested && M.cls == (int)c;
-        if (n == 0) continue;
+        bool any = false;
+        for (const EngMember &M : e->members) any = any || (M.used && !M.done && !M.nested && M.cls == (int)c);
+        if (!any) continue;
         GcFusedGrid g;
         memset(&g, 0, sizeof g);
         g.nx = e->classes[c].nx; g.ny = e->classes[c].ny; g.pitch = e->classes[c].pitch;
         gc_block_plan(e->block_variant, g, e->block_T);
-        if (!gc_block_fits(g, n)) return false;
+        if (!gc_block_fits(g, 1)) return false;
     }
     return true;
 }
@@ -625,6 +625,8 @@ static int eng_rebuild(gc_engine *e) {
         for (int g = 1; g < e->ngrids && same; g++)
             same = grids[g].nx == grids[0].nx && grids[g].ny == grids[0].ny && grids[g].pitch == grids[0].pitch &&
                    grids[g].rows == grids[0].rows;
+        /* a work list where the class launch's window numbers do not fit */
+        if (e->block_now && !gc_block_fits(grids[0], e->ngrids)) same = false;
         if (same) {
             memset(&e->pcls, 0, sizeof e->pcls);
             e->pcls.proto = grids[0];

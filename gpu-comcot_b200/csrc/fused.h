@@ -153,7 +153,8 @@ int gc_block_num_forms();
 void gc_block_form(int form, int *variant, int *steps);
 int gc_block_pick_form(int ngrids, const int *nx, const int *ny);
 /* whether a planned grid's byte offsets and window numbers fit 32 bits
- * (`members` of them in a class launch) */
+ * (`members` of them in a class launch; 1 in a launch of one grid or of a
+ * work list, which divides no window number by the members) */
 bool gc_block_fits(const GcFusedGrid &g, int members);
 /* diagnostics: the bytes of a field from which on a grid does not fit (at most
  * 4 GB, where its offsets run out; <= 0 restores that) */
