@@ -63,7 +63,7 @@ struct Staging {
             bool own = false;
             for (int k = 1; k >= 0; k--) {
                 if (busy[k] && cudaEventQuery(busy[k]) == cudaErrorNotReady) {
-                    cudaGetLastError(); /* an answer, not an error */
+                    if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError(); /* an answer, not an error */
                     own = own || by[k] == s;
                     continue;
                 }

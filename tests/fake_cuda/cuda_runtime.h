@@ -50,6 +50,7 @@ inline std::mutex mu;
 inline std::condition_variable cv;
 inline std::map<const char *, std::pair<size_t, cudaMemoryType>> known; /* start -> size, kind */
 inline thread_local int device = 0;
+inline thread_local cudaError_t last = cudaSuccess;
 inline int device_callers = 0; /* copies whose caller's side is device memory */
 
 inline cudaMemoryType kind(const void *p) {
@@ -87,7 +88,12 @@ inline void set_open(FakeStream *s, bool open) {
 } // namespace fake
 
 inline const char *cudaGetErrorString(cudaError_t) { return "fake CUDA error"; }
-inline cudaError_t cudaGetLastError() { return cudaSuccess; }
+inline cudaError_t cudaPeekAtLastError() { return fake::last; }
+inline cudaError_t cudaGetLastError() {
+    const cudaError_t e = fake::last;
+    fake::last = cudaSuccess;
+    return e;
+}
 inline cudaError_t cudaGetDevice(int *d) { *d = fake::device; return cudaSuccess; }
 inline cudaError_t cudaSetDevice(int d) { fake::device = d; return cudaSuccess; }
 inline cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
@@ -124,7 +130,9 @@ inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
 inline cudaError_t cudaEventQuery(cudaEvent_t e) {
     std::unique_lock<std::mutex> l(fake::mu);
     if (e->stream && e->stream->open) fake::drain(l, e->stream, e->at);
-    return !e->stream || e->stream->ran >= e->at ? cudaSuccess : cudaErrorNotReady;
+    if (!e->stream || e->stream->ran >= e->at) return cudaSuccess;
+    if (fake::last == cudaSuccess) fake::last = cudaErrorNotReady;
+    return cudaErrorNotReady;
 }
 inline cudaError_t cudaEventSynchronize(cudaEvent_t e) {
     std::unique_lock<std::mutex> l(fake::mu);
