@@ -45,9 +45,10 @@ struct GcFusedGrid {
     const float *gw;    /* [2*ng] (CX, CY) */
     float *ts;
     int ts_len;         /* steps the ts buffer can hold */
-    /* when has_win: cells [wi0,wi1] x [wj0,wj1] (0-based, inclusive) get no
-     * max-eta or arrival update, since a nested child's feedback rewrites
-     * their surface after this launch (zero-filled descriptors have none) */
+    /* kernels_step.cu alone, when has_win: cells [wi0,wi1] x [wj0,wj1]
+     * (0-based, inclusive) get no max-eta or arrival update, since a nested
+     * child's feedback rewrites their surface after this launch (zero-filled
+     * descriptors have none) */
     int has_win, wi0, wi1, wj0, wj1;
     /* register-tile kernel: margin rows of a window (the most steps a launch
      * may take), windows along I and J, windows on the perimeter (numbered

@@ -481,8 +481,7 @@ __device__ __forceinline__ void block_run(const Desc &G, BlockSmem<R, NW> &S, co
                         for (int k = 0; k < 4; k++) {
                             const int i = W.ib + k;
                             if (zv[k] > thr && xv[k] <= thr && (W.wc >> (4 * r + k) & 1) && j >= q.jlo && j <= q.jhi &&
-                                i >= q.lo && i <= q.hi &&
-                                !(G.has_win && i >= G.wi0 && i <= G.wi1 && j >= G.wj0 && j <= G.wj1))
+                                i >= q.lo && i <= q.hi)
                                 row[i] = local + t + 1;
                         }
                     }
@@ -709,8 +708,6 @@ __device__ __forceinline__ void block_tile(const Desc &G, int lt, int step, int 
     unsigned o = (unsigned)W.jw * p4 + 4u * (unsigned)W.ib;
     char *zo = (char *)G.z[wr], *mo = (char *)G.m[wr], *no = (char *)G.n[wr], *xo = (char *)G.zmax;
     const bool whole = W.ib >= q.lo && W.ib + 3 <= q.hi, part = !whole && W.ib + 3 >= q.lo && W.ib <= q.hi;
-    /* max-eta is left to the child's feedback inside its window */
-    const bool xplain = do_max && !(G.has_win && q.s <= G.wi1 && q.s + BW > G.wi0 && q.sj <= G.wj1 && q.sj + RW > G.wj0);
 #pragma unroll
     for (int r = 0; r < R; r++, o += p4) {
         const int j = W.jw + r;
@@ -719,9 +716,9 @@ __device__ __forceinline__ void block_tile(const Desc &G, int lt, int step, int 
             *(float4 *)(zo + o) = f4(z[r]);
             *(float4 *)(mo + o) = f4(m[r]);
             *(float4 *)(no + o) = f4(n[r]);
-            if (xplain) *(float4 *)(xo + o) = f4(x[r]);
+            if (do_max) *(float4 *)(xo + o) = f4(x[r]);
         }
-        if (part || (whole && do_max && !xplain)) {
+        if (part) {
             const float4 zv = f4(z[r]), mv = f4(m[r]), nv = f4(n[r]), xv = f4(x[r]);
             const float zz[4] = {zv.x, zv.y, zv.z, zv.w}, mm[4] = {mv.x, mv.y, mv.z, mv.w};
             const float nn[4] = {nv.x, nv.y, nv.z, nv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
@@ -729,13 +726,10 @@ __device__ __forceinline__ void block_tile(const Desc &G, int lt, int step, int 
             for (int k = 0; k < 4; k++) {
                 const int i = W.ib + k;
                 if (i < q.lo || i > q.hi) continue;
-                if (part) {
-                    *(float *)(zo + o + 4 * k) = zz[k];
-                    *(float *)(mo + o + 4 * k) = mm[k];
-                    *(float *)(no + o + 4 * k) = nn[k];
-                }
-                if (do_max && !(G.has_win && i >= G.wi0 && i <= G.wi1 && j >= G.wj0 && j <= G.wj1))
-                    *(float *)(xo + o + 4 * k) = xx[k];
+                *(float *)(zo + o + 4 * k) = zz[k];
+                *(float *)(mo + o + 4 * k) = mm[k];
+                *(float *)(no + o + 4 * k) = nn[k];
+                if (do_max) *(float *)(xo + o + 4 * k) = xx[k];
             }
         }
     }
@@ -745,7 +739,7 @@ __device__ __forceinline__ void block_tile(const Desc &G, int lt, int step, int 
 struct BlockClassDesc {
     const int &nx, &ny, &pitch, &bt, &bntx, &bnty, &bper;
     const unsigned &bmag;
-    const int &nbuf, &cur0, &has_win, &wi0, &wi1, &wj0, &wj1;
+    const int &nbuf, &cur0;
     const float *const &rows;
     float *const (&z)[3];
     float *const (&m)[3];
@@ -759,10 +753,9 @@ struct BlockClassDesc {
     const int &step0, &nsteps, &flags, &ng;
     const float &thr;
     __device__ __forceinline__ BlockClassDesc(const GcFusedGrid &p, const GcPairMember &q)
-        : nx(p.nx), ny(p.ny), pitch(p.pitch), bt(p.bt), bntx(p.bntx), bnty(p.bnty), bper(p.bper), bmag(p.bmag), nbuf(p.nbuf), cur0(p.cur0), has_win(p.has_win), wi0(p.wi0),
-          wi1(p.wi1), wj0(p.wj0), wj1(p.wj1), rows(p.rows), z(q.z), m(q.m), n(q.n), zmax(q.zmax), arrival(q.arrival),
-          h(q.h), gij(q.gij), gw(q.gw), ts(q.ts), step0(q.step0), nsteps(q.nsteps), flags(q.flags), ng(q.ng),
-          thr(q.thr) {}
+        : nx(p.nx), ny(p.ny), pitch(p.pitch), bt(p.bt), bntx(p.bntx), bnty(p.bnty), bper(p.bper), bmag(p.bmag),
+          nbuf(p.nbuf), cur0(p.cur0), rows(p.rows), z(q.z), m(q.m), n(q.n), zmax(q.zmax), arrival(q.arrival), h(q.h),
+          gij(q.gij), gw(q.gw), ts(q.ts), step0(q.step0), nsteps(q.nsteps), flags(q.flags), ng(q.ng), thr(q.thr) {}
 };
 
 /* one window per CTA: edge windows last longer, and the hardware hands the

@@ -335,11 +335,8 @@ __device__ __forceinline__ bool warp_tile(const GcFusedGrid &Gref, int lt, int s
     float *n2p = n2 + (size_t)j0 * P + ib;
 
     /* a tile none of whose cells (halo row and column included) lies on a
-     * grid edge or in the max/arrival exclusion window runs a body compiled
-     * without any boundary logic */
-    const int wi0 = Gref.wi0, wi1 = Gref.wi1, wj0 = Gref.wj0, wj1 = Gref.wj1;
-    const bool inwin = Gref.has_win && i0 <= wi1 && i0 + TXW - 1 >= wi0 && j0 <= wj1 && j0 + TY - 1 >= wj0;
-    const bool edge = inwin || !(i0 >= 1 && i0 + TXW <= nx - 2 && j0 >= 1 && j0 + TY <= ny - 2);
+     * grid edge runs a body compiled without any boundary logic */
+    const bool edge = !(i0 >= 1 && i0 + TXW <= nx - 2 && j0 >= 1 && j0 + TY <= ny - 2);
     /* FL_NC: N of rows r-1 (this row's stage B) and r-2 (carried) at columns c0..c0+4 */
     float nbk[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, nck[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
     for (int k = 1; k <= TY + 1 && ok; k++) {
@@ -421,13 +418,6 @@ __device__ __forceinline__ bool warp_tile(const GcFusedGrid &Gref, int lt, int s
                 if (k <= TY && own) {
                     if constexpr (EDGE) st4p(z2p, ib, nx, zn);
                     else *reinterpret_cast<float4 *>(z2p) = make_float4(zn[0], zn[1], zn[2], zn[3]);
-                    /* cells whose surface a child's feedback rewrites later */
-                    bool skip[4] = {false, false, false, false};
-                    if constexpr (EDGE) {
-#pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            skip[q] = inwin && r >= wj0 && r <= wj1 && ib + q >= wi0 && ib + q <= wi1;
-                    }
                     float xo[4] = {0.0f, 0.0f, 0.0f, 0.0f}; /* max-eta before this step */
                     if (do_max) {
                         float4 x4;
@@ -436,7 +426,7 @@ __device__ __forceinline__ bool warp_tile(const GcFusedGrid &Gref, int lt, int s
                         xo[0] = x4.x; xo[1] = x4.y; xo[2] = x4.z; xo[3] = x4.w;
                         float zx[4];
 #pragma unroll
-                        for (int q = 0; q < 4; q++) zx[q] = (xo[q] >= zn[q] || skip[q]) ? xo[q] : zn[q];
+                        for (int q = 0; q < 4; q++) zx[q] = xo[q] >= zn[q] ? xo[q] : zn[q];
                         if constexpr (EDGE) st4p(zxp, ib, nx, zx);
                         else *reinterpret_cast<float4 *>(zxp) = make_float4(zx[0], zx[1], zx[2], zx[3]);
                     }
@@ -445,7 +435,7 @@ __device__ __forceinline__ bool warp_tile(const GcFusedGrid &Gref, int lt, int s
                         if (zhi > thr) {
 #pragma unroll
                             for (int q = 0; q < 4; q++) {
-                                if (ib + q < nx && zn[q] > thr && hv[q] > CC_GX && !skip[q]) {
+                                if (ib + q < nx && zn[q] > thr && hv[q] > CC_GX) {
                                     int *a = arrival + (size_t)r * P + ib + q;
                                     /* GC_F_ARR_BYMAX: max-eta has taken every step
                                      * since the start, so a wet cell whose max so
