@@ -8,8 +8,8 @@
  * (GPUOutput.cu:46-53), the arrival record and the gauge samples (GET_TS,
  * output.f90:1078-1090) of every step.
  *
- * Work decomposition: a CTA of NW warps owns a window of 64 columns x
- * RW = R*NW rows.  A lane owns two adjacent columns of R rows and keeps
+ * Work decomposition: a CTA of NW warps owns a window of 128 columns x
+ * RW = R*NW rows.  A lane owns four adjacent columns of R rows and keeps
  * their Z, M, N and max-eta in registers from the first step of the launch
  * to the last; a warp's R rows lie under the next warp's.  Neighbours along
  * I are warp shuffles, neighbours along J are the lane's own registers, and
@@ -17,12 +17,13 @@
  * shared memory, once per step.  A step's result is exact where the previous
  * step was exact one cell further out, so after T steps a margin of T cells
  * at each side of the window is stale: windows overlap by it (by T rounded
- * up to even along I, which keeps every lane's pair 8-byte aligned) and only
- * the core is stored.  At the grid's own edges there is no margin: the
- * perimeter takes OPEN and the clamps, which read nothing beyond it.
+ * up to a multiple of 4 along I, so that a lane lies in the margin or outside
+ * it as a whole and its loads and stores stay 16-byte aligned) and only the
+ * core is stored.  At the grid's own edges there is no margin: the perimeter
+ * takes OPEN and the clamps, which read nothing beyond it.
  *
- * Arithmetic: the two columns of a lane are the two halves of one packed
- * operation (add/sub/mul .rn.f32x2, each half rounded separately), except
+ * Arithmetic: the four columns of a lane are the halves of two packed
+ * operations (add/sub/mul .rn.f32x2, each half rounded separately), except
  * where an operand is shifted by one column.  The order of operations is the
  * Fortran's, so the results are the bits of T launches of the one-step kernel.
  *
@@ -36,24 +37,29 @@
  * window last three times an inner one.  A warp whose water is still in every
  * reach of the step computes nothing for that step.
  *
- * What bounds it (ncu, 2401 x 2001, 32-row windows, 4 steps): the FMA pipe
- * carries two thirds of the instructions (a packed operation holds it for two
- * cycles; the Fortran order allows no fused multiply-add), 43 % of the issue
- * slots are busy with 14 warps per SM, DRAM is at a third of its rate.  Four
- * columns a lane against two (64-column windows) halved the shared-memory
- * exchange and the shuffles per cell.
+ * What bounds it (ncu, 2401 x 2001, waves everywhere, 64-row windows, 8
+ * steps): no unit is full.  46 % of the issue slots are busy with 15.5 warps
+ * an SM (128 registers a thread), the FMA pipe 28 % and the ALU pipe 35 % of
+ * the cycles, DRAM 9 % of its rate.  Per issued instruction a warp waits 1.4
+ * cycles for a math pipe (a packed operation holds it for two cycles), 1.4 for
+ * a fixed latency, 1.0 at the step's barrier and 0.7 for shared memory.  Its
+ * 924 windows are 6.2 waves of one CTA an SM, so 14 % of the time is the last
+ * wave.
  *
- * Time per step, one grid, against the two-step kernel (kernels_pair.cu) on
- * the same B200, waves everywhere: 361 x 301 2.5 us against 8.2, 961 x 801
- * 4.4 against 10.0, 1201 x 1001 5.6 against 12.2, 2401 x 2001 19.5 against
- * 22.4; eight grids of 1201 x 1001 38.7 against 56.6.  A young forecast, its
- * wave in one corner of 2401 x 2001: 10.4 against 22.2.
+ * Time per step of eager launches, waves everywhere, against the two-step
+ * kernel (kernels_pair.cu) on the same B200: 361 x 301 2.8 us against 8.3,
+ * 961 x 801 4.6 against 9.8, 1201 x 1001 5.6 against 11.6, 2401 x 2001 19.1
+ * against 22.1, eight grids of 1201 x 1001 39 against 47; of 64 such grids
+ * with waves everywhere the two-step kernel is ahead, 303 against 309.  Young
+ * forecasts, their waves in one corner: 2401 x 2001 11.2 against 21.4, 64 of
+ * 1201 x 1001 230 against 302.
  *
- * Tried and measured slower on 2401 x 2001: a persistent form with the next
- * window's fields fetched by tensor copies into shared memory while this one
- * steps, results out by tensor copies (12 warps per SM, 24 us per step: the
- * buffers cost the warps that hide latency); 1-D copies issued by every lane
- * (200 copies a window, 24 cycles each, 26 us).
+ * Tried and measured slower on 2401 x 2001 with 4 steps a launch: 64 columns a
+ * window and two a lane (35 us a step, with twice the exchange and shuffles a
+ * cell); a persistent form with the next window's fields fetched by tensor
+ * copies into shared memory while this one steps, results out by tensor copies
+ * (12 warps an SM, 24 us: the buffers cost the warps that hide latency); 1-D
+ * copies issued by every lane (200 copies a window, 24 cycles each, 26 us).
  *
  * No copy engine and no waits on memory barriers of its own: plain loads, all
  * of a window's rows in flight at once, and CTA barriers.
@@ -874,8 +880,8 @@ int gc_block_plan(int variant, GcFusedGrid &g, int bt) {
  * timed runs with waves everywhere on one grid of 361 x 301 to 2401 x 2001
  * cells and on 8 and 24 grids of 1201 x 1001 (within 15 % of most).  Small
  * grids want many small windows, large ones windows with little margin: per
- * step, 2.5 us (24 rows, 8 steps) against 4.6 us (64 rows) at 361 x 301, and
- * 48.3 us against 19.5 us at 2401 x 2001. */
+ * step, 2.8 us (24 rows, 8 steps) against 5.3 us (64 rows) at 361 x 301, and
+ * 46 us against 19.1 us at 2401 x 2001. */
 struct BlockForm {
     int variant, steps, per_sm;
     float lone, a, b;

@@ -38,6 +38,11 @@
  * tile reads (the one-step kernel writes L + 1 the same way).  Level L + 1 is
  * never stored.
  *
+ * The register-tile kernel (kernels_block.cu) is ahead nearly everywhere.  This
+ * one serves grids with fields of 4 GB and more, whose offsets do not fit that
+ * kernel's 32 bits, and stays a candidate of the autotuner: 64 grids of
+ * 1201 x 1001 with waves everywhere take 303 us a step here and 309 there.
+ *
  * Every pipeline wait is bounded by the `wait_limit` launch parameter; a wait
  * that gives up sets g_pair_error and the warp leaves once its copies in
  * flight have landed (or a second bounded wait expired).  `stall` != 0 makes

@@ -593,13 +593,10 @@ __device__ __forceinline__ bool adv_span(int i, int j, int ix, int jy) {
 }
 
 /* CONMOME, one face per thread, the x and y directions as two grid layers.
- * Every value a face can need (its stencil reaches two cells back along the
- * face normal's neighbour axis and one cell forward) is loaded first, as
- * one batch of independent loads at clamped, in-bounds indices; the
- * branches then run on registers.  Clamped indices coincide with the
- * reference's wherever a value is used: the two-back neighbours are read
- * only inside the advection span, whose cells are at least 10 from every
- * edge. */
+ * conmome_face reads the fields where it needs them, the advection stencil
+ * inside its branches, at clamped, in-bounds indices, which coincide with the
+ * reference's wherever a value is used: the two-back neighbours are read only
+ * inside the advection span, whose cells are at least 10 from every edge. */
 template <bool SPH>
 __global__ void k_conmome(GcLayerDev L, int upd) {
     pdl_enter();
@@ -644,7 +641,7 @@ __global__ void k_conmome(GcLayerDev L, int upd) {
  * N (two cells of halo, at the same clamped indices the one-face kernel
  * reads) with one batch of independent loads, then each thread computes
  * its cell's x and y faces from shared memory.  Same values, same
- * arithmetic (conmome_x / conmome_y): the same bits. */
+ * arithmetic (conmome_face): the same bits. */
 template <bool SPH, int TY>
 __device__ __forceinline__ void conmome_tile_body(const GcLayerDev &L, int upd) {
     pdl_enter();
