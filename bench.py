@@ -276,30 +276,25 @@ def timed_engine_steps(torch, eng, steps, warmup, dist, local):
     return ms, launches, ck
 
 
-BLOCK_FORMS = 8  # the last candidates: the register-tile kernel's forms
-
-
-def steps_per_launch(variant, steps, launches):
-    """steps per launch of the timed window: 1 for the one-step kernel's
-    candidates, 2 for the two-step kernel's after them, and as counted for the
-    register-tile kernel's, whose launches take up to 4 or 8"""
+def candidate_kernel(variant):
+    """the step kernel of an engine candidate: "fused" (one step a launch),
+    "pair" (two) or "block" (the register-tile kernel, up to 4 or 8)"""
     from comcot_b200 import _lib
 
     lib = _lib.load()
-    if variant >= lib.gc_engine_num_candidates() - BLOCK_FORMS:
-        return steps / max(1, launches)
-    return 2 if variant >= 2 * lib.gc_engine_num_variants() else 1
+    if variant >= lib.gc_engine_num_candidates() - lib.gc_engine_num_block_forms():
+        return "block"
+    return "pair" if variant >= 2 * lib.gc_engine_num_variants() else "fused"
+
+
+def steps_per_launch(variant, steps, launches):
+    """steps per launch of the timed window, counted where it varies"""
+    return {"fused": 1, "pair": 2, "block": steps / max(1, launches)}[candidate_kernel(variant)]
 
 
 def profile_name(kind, variant):
     """the committed counter summary of the candidate's kernel"""
-    from comcot_b200 import _lib
-
-    lib = _lib.load()
-    step = {"linear": "linear_step_c2.txt", "ensemble": "ensemble_step_c4.txt"}[kind]
-    if variant >= lib.gc_engine_num_candidates() - BLOCK_FORMS:
-        return "block_" + step
-    return ("pair_" if variant >= 2 * lib.gc_engine_num_variants() else "fused_") + step
+    return f"{candidate_kernel(variant)}_" + {"linear": "linear_step_c2.txt", "ensemble": "ensemble_step_c4.txt"}[kind]
 
 
 def merge_parity(records):
@@ -756,7 +751,8 @@ def run_single(args, torch, dist, rank, world, local):
     # candidates of several steps a launch run whole launches (8 steps at most);
     # the second round re-times the three fastest over three 64-step graph
     # chunks each
-    total = (ncand - BLOCK_FORMS) * (2 * tune_reps + 2) + BLOCK_FORMS * 8 * (tune_reps + 1) + 3 * 3 * 64 \
+    nblock = lib.gc_engine_num_block_forms()
+    total = (ncand - nblock) * (2 * tune_reps + 2) + nblock * 8 * (tune_reps + 1) + 3 * 3 * 64 \
         + args.warmup + args.steps + 8
     make_case = synth.config_c1 if args.workload == "c1" else synth.config_c2
     case = make_case(nsteps=total)

@@ -1410,6 +1410,7 @@ int gc_engine_variant(gc_engine *e) {
 }
 int gc_engine_num_variants(void) { return gc_fused_num_variants(); }
 int gc_engine_num_candidates(void) { return eng_num_candidates(); }
+int gc_engine_num_block_forms(void) { return gc_block_num_forms(); }
 
 void *gc_engine_stream(gc_engine *e) { return e ? (void *)e->stream : nullptr; }
 long long gc_engine_launches(gc_engine *e) { return e ? e->launches : GC_EINVAL; }

@@ -84,17 +84,17 @@ def test_autotuner_leaves_out_what_does_not_fit(low_limit):
         eng.add(case)
         best = eng.autotune(1)
         eng.step(1)
-        assert 0 <= best < ncand - 8 and eng.variant() == best
+        assert 0 <= best < ncand - low_limit.gc_engine_num_block_forms() and eng.variant() == best
 
 
 def test_a_long_work_list_keeps_its_steps_a_launch(oracle_mod):
     """13500 grids: the square of their number, which only a class launch (at most 48) divides by, is beyond 32 bits
     times the windows of one"""
-    n, steps = 13500, 8
+    lib, n, steps = _lib.load(), 13500, 8
     case = synth.single_layer_case("w", 3, 200, 2.0, 2.0, steps, seed=4, n_seamounts=0, shelf_cols=1, land_cols=0,
                                    source="hump", amp=2.0)
     with Engine(budget=8 << 30) as eng:
-        eng.config(variant=_lib.load().gc_engine_num_candidates() - 8, use_graphs=0)   # 16 rows a window, 4 steps a launch
+        eng.config(variant=lib.gc_engine_num_candidates() - lib.gc_engine_num_block_forms(), use_graphs=0)   # 16 rows a window, 4 steps a launch
         cls = eng.add_class(case.root)
         ids = [eng.add(case, cls=cls) for _ in range(n)]
         eng.step(steps + 1)
