@@ -94,15 +94,14 @@ def profiled_traffic(name="fused_linear_step_c2.txt", key="traffic_bytes_per_lau
 
 def pair_note(rl, one_step_gbs):
     """a launch of several steps reads and writes each cell once for all of
-    them, so its HBM fraction is of a part of the one-step bytes; it is bounded
-    by the arithmetic pipes and instruction issue instead.  Adds the HBM
+    them, so its HBM fraction is of a part of the one-step bytes.  Adds the HBM
     fraction a one-step kernel would need for the same steps/s, and the
     limiter."""
     if rl.get("steps_per_launch") > 1:
         rl["one_step_equivalent_gbs"] = one_step_gbs
         rl["one_step_equivalent_frac"] = one_step_gbs / rl["peak"]
-        rl["limiter"] = ("FMA pipe and instruction issue (several steps per HBM pass: same bytes per launch as one "
-                         "step); figures in the kernel's summary under profiles/")
+        rl["limiter"] = ("not HBM: several steps per pass over it, the same bytes per launch as one step; what bounds "
+                         "the kernel is in its summary under profiles/")
     return rl
 
 
@@ -737,6 +736,34 @@ def run_c5(args, torch, dist, rank, world, local):
 # ---------------------------------------------------------------------------
 # C1 / C2: one grid (the headline)
 # ---------------------------------------------------------------------------
+def moving_water(torch, workload, variant, steps=256, warmup=1024):
+    """Per-step time of the workload's grid with waves on every wet cell: the
+    register-tile kernel computes nothing for rows whose water is still, as
+    most of a young forecast's is, so its headline rate counts cells that took
+    no arithmetic; here every cell takes it.  The warm-up is long enough for
+    most arrivals to lie behind."""
+    from comcot_b200.engine import Engine
+
+    case = (synth.config_c1 if workload == "c1" else synth.config_c2)(nsteps=steps + warmup)
+    L = case.root
+    j, i = np.mgrid[0:L.ny, 0:L.nx]
+    L.Z0 = np.where(L.H > 0, 0.3 * np.sin(0.11 * i + 0.07 * j), 0.0).astype(np.float32)
+    with Engine(budget=8 << 30) as eng:
+        eng.config(variant=variant, use_graphs=1, chunk=64)
+        eng.add(case)
+        eng.prepare()
+        eng.step(warmup)
+        eng.sync()
+        stream = torch.cuda.ExternalStream(eng.stream())
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(stream)
+        eng.step(steps)
+        b.record(stream)
+        b.synchronize()
+        ms = a.elapsed_time(b) / steps
+    return {"value": L.nx * L.ny / (ms * 1e-3), "unit": METRIC, "ms_per_step": ms, "steps": steps, "n_gpus": 1}
+
+
 def run_single(args, torch, dist, rank, world, local):
     """C1 / C2: one linear spherical grid (value: the engine, device-resident;
     e2e: the reference C ABI with host buffers over one whole forecast;
@@ -772,6 +799,8 @@ def run_single(args, torch, dist, rank, world, local):
     done = eng.steps_done(mid)
     got = eng.read(mid)
     eng.close()
+    # the same with no still water for the step kernel to leave out
+    moving = moving_water(torch, args.workload, variant)
 
     # ---------------- end to end through the reference C ABI ----------------
     e2e, e2e_state = None, None
@@ -829,6 +858,7 @@ def run_single(args, torch, dist, rank, world, local):
                               achieved * spl),
         "clocks": ck,
         "gpu_launches": launches,
+        "waves_everywhere": moving,
     }
     if e2e:
         line["e2e"] = e2e
