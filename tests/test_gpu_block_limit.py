@@ -88,8 +88,8 @@ def test_autotuner_leaves_out_what_does_not_fit(low_limit):
 
 
 def test_a_long_work_list_keeps_its_steps_a_launch(oracle_mod):
-    """13500 grids: the square of their number, which only a class launch (at most 48) divides by, is beyond 32 bits
-    times the windows of one"""
+    """13500 grids: the windows of one times the square of their number, the bound of a class launch (at most 64
+    members), is beyond 32 bits"""
     lib, n, steps = _lib.load(), 13500, 8
     case = synth.single_layer_case("w", 3, 200, 2.0, 2.0, steps, seed=4, n_seamounts=0, shelf_cols=1, land_cols=0,
                                    source="hump", amp=2.0)
