@@ -140,12 +140,12 @@ void gc_copy(void *dst, const void *src, size_t bytes) {
         memcpy((char *)dst + a, (const char *)src + a, b - a);
     };
     std::vector<std::thread> pool;
-    pool.reserve(nt);
     int started = 1;
     try {
+        pool.reserve(nt);
         for (; started < nt; started++) pool.emplace_back(work, started);
     } catch (...) {
-        /* no more threads: this one copies the rest */
+        /* no more threads, or no memory for them: this one copies the rest */
         for (int t = started; t < nt; t++) work(t);
     }
     work(0);

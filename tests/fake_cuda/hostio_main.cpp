@@ -5,7 +5,17 @@
 #include <stdio.h>
 #include <unistd.h>
 
+#include <new>
 #include <string>
+
+static thread_local bool out_of_memory = false;
+void *operator new(size_t n) {
+    void *p = out_of_memory ? nullptr : malloc(n);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
 
 namespace {
 
@@ -115,6 +125,17 @@ int device_caller(int nx, int ny) {
     return 0;
 }
 
+/* a copy that can have no threads is made by its caller */
+int no_memory(size_t bytes) {
+    std::vector<char> a(bytes), b(bytes);
+    for (size_t k = 0; k < bytes; k++) a[k] = (char)(k * 7 + k / 251);
+    out_of_memory = true;
+    const int rc = gc_host_copy(b.data(), a.data(), (long long)bytes);
+    out_of_memory = false;
+    CHECK(rc == GC_OK && a == b);
+    return 0;
+}
+
 } // namespace
 
 int main(int argc, char **argv) {
@@ -129,6 +150,7 @@ int main(int argc, char **argv) {
     if (what == "beside-upload") return beside(nx, ny, 2, false);
     if (what == "foreign-device") return foreign(nx, ny);
     if (what == "device-caller") return device_caller(nx, ny);
+    if (what == "no-memory") return no_memory((size_t)9 << 20);
     printf("no scenario %s\n", what.c_str());
     return 2;
 }

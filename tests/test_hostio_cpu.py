@@ -45,3 +45,7 @@ def test_transfers_on_a_device_that_is_not_current(scenario, nx, ny):
 @pytest.mark.parametrize("nx,ny", [(33, 17), (300, 300), (2401, 2001)])
 def test_callers_device_memory_is_left_to_the_runtime(scenario, nx, ny):
     scenario("device-caller", nx, ny)
+
+
+def test_copy_without_memory_for_threads(scenario):
+    scenario("no-memory")
