@@ -799,9 +799,6 @@ def run_single(args, torch, dist, rank, world, local):
     done = eng.steps_done(mid)
     got = eng.read(mid)
     eng.close()
-    # the same with no still water for the step kernel to leave out
-    moving = moving_water(torch, args.workload, variant)
-
     # ---------------- end to end through the reference C ABI ----------------
     e2e, e2e_state = None, None
     E = FORECAST_STEPS[args.workload]
@@ -836,6 +833,9 @@ def run_single(args, torch, dist, rank, world, local):
                         "stencils gathered on the device, update; stencils read back once per 1024 steps) "
                         "+ getz/getzmax")}
         s.close()
+
+    # the step rate with no still water for the kernel to leave out
+    moving = moving_water(torch, args.workload, variant)
 
     peak, peak_kind = peaks()
     spl = steps_per_launch(variant, args.steps, launches)
