@@ -16,8 +16,9 @@
  * its buffers and returns.  A call that finds too few buffers free because
  * another stream's uploads are still queued takes the plain copy, so no caller
  * waits for another one's steps; so do smaller transfers, those whose caller's
- * side is device memory, which host threads cannot touch, and all where the
- * buffers cannot be had.
+ * side is not ordinary memory (page-locked memory needs no staging, device
+ * memory no host thread can touch, and both may be what earlier work on the
+ * stream writes or reads), and all where the buffers cannot be had.
  */
 #include <string.h>
 
@@ -114,14 +115,14 @@ bool capturing(cudaStream_t s) {
     return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
 }
 
-/* Whose memory a caller's pointer names.  An asynchronous copy from ordinary
- * host memory has read it when the call returns, while one from page-locked,
- * managed or device memory reads it when the stream gets there. */
-cudaMemoryType memory_of(const void *p) {
+/* Ordinary host memory: an asynchronous copy from it has read it when the call
+ * returns, while one from page-locked, managed or device memory reads it when
+ * the stream gets there, after what earlier work on the stream writes to it. */
+bool pageable(const void *p) {
     cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    return cudaMemoryTypeHost; /* unknown: waited for */
+    return false; /* unknown: the plain copy, waited for */
 }
 
 } // namespace
@@ -157,15 +158,15 @@ int gc_field_upload(float *d, size_t pitch_bytes, const float *h, int nx, int ny
     std::unique_lock<std::mutex> lock(g_staging.mu, std::defer_lock);
     int first = -1;
     const bool capture = capturing(s);
-    const cudaMemoryType from = memory_of(h);
-    if (total >= kSmall && row <= kSlot && !capture && from != cudaMemoryTypeDevice) {
+    const bool host = pageable(h);
+    if (total >= kSmall && row <= kSlot && !capture && host) {
         const int rows = (int)(kSlot / row), pieces = (ny + rows - 1) / rows;
         if (pieces > 2) GC_CUDA_OR_RET(cudaStreamSynchronize(s)); /* the third piece waits for the first copy */
         first = g_staging.take(lock, std::min(pieces, 2), s);
     }
     if (first < 0) {
         GC_CUDA_OR_RET(cudaMemcpy2DAsync(d, pitch_bytes, h, row, row, (size_t)ny, cudaMemcpyHostToDevice, s));
-        if (from != cudaMemoryTypeUnregistered && !capture) GC_CUDA_OR_RET(cudaStreamSynchronize(s));
+        if (!host && !capture) GC_CUDA_OR_RET(cudaStreamSynchronize(s));
         return GC_OK;
     }
     const int rows = (int)(kSlot / row);
@@ -186,7 +187,7 @@ int gc_field_download(void *h, const void *d, size_t pitch_bytes, int nx, int ny
     const size_t row = (size_t)nx * sizeof(float), total = row * ny;
     std::unique_lock<std::mutex> lock(g_staging.mu, std::defer_lock);
     int first = -1;
-    if (total >= kSmall && row <= kSlot && !capturing(s) && memory_of(h) != cudaMemoryTypeDevice) {
+    if (total >= kSmall && row <= kSlot && !capturing(s) && pageable(h)) {
         GC_CUDA_OR_RET(cudaStreamSynchronize(s));
         first = g_staging.take(lock, 2, s);
     }

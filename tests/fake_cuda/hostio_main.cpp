@@ -125,6 +125,24 @@ int device_caller(int nx, int ny) {
     return 0;
 }
 
+/* memory that work on the stream writes before an upload or reads after a
+ * download: the transfer is in stream order, not ahead of it */
+int ordered(int nx, int ny, cudaMemoryType kind) {
+    FakeStream s;
+    Field f(nx, ny, 5.0f);
+    const size_t bytes = f.host.size() * sizeof(float);
+    float *h = (float *)fake::make(bytes, kind);
+    fake::push(&s, [&] { memcpy(h, f.host.data(), bytes); });
+    CHECK(gc_field_upload(f.dev, f.row(), h, nx, ny, &s) == GC_OK);
+    CHECK(cudaStreamSynchronize(&s) == cudaSuccess && f.there(f.host.data()));
+    std::vector<float> seen(f.host.size());
+    memset(h, 0xff, bytes);
+    fake::push(&s, [&] { memcpy(seen.data(), h, bytes); });
+    CHECK(gc_field_download(h, f.dev, f.row(), nx, ny, &s) == GC_OK && memcmp(h, f.host.data(), bytes) == 0);
+    CHECK(memcmp(seen.data(), f.host.data(), 4) != 0); /* the reader that came first saw what was there */
+    return 0;
+}
+
 /* a copy that can have no threads is made by its caller */
 int no_memory(size_t bytes) {
     std::vector<char> a(bytes), b(bytes);
@@ -150,6 +168,9 @@ int main(int argc, char **argv) {
     if (what == "beside-upload") return beside(nx, ny, 2, false);
     if (what == "foreign-device") return foreign(nx, ny);
     if (what == "device-caller") return device_caller(nx, ny);
+    if (what == "ordered-locked") return ordered(nx, ny, cudaMemoryTypeHost);
+    if (what == "ordered-managed") return ordered(nx, ny, cudaMemoryTypeManaged);
+    if (what == "ordered-device") return ordered(nx, ny, cudaMemoryTypeDevice);
     if (what == "no-memory") return no_memory((size_t)9 << 20);
     printf("no scenario %s\n", what.c_str());
     return 2;

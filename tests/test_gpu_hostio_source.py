@@ -47,3 +47,29 @@ def test_setters_read_before_they_return(nx, ny, locked):
         s.close()
         for p in ptrs:
             lib.gc_host_free(p)
+
+
+@pytest.mark.parametrize("nx,ny", [(200, 200), (300, 300)])
+def test_setter_follows_work_on_the_librarys_stream(nx, ny):
+    """page-locked memory that queued work on the library's stream fills"""
+    lib = _lib.load()
+    case = synth.single_layer_case("o", nx, ny, 2.0, 2.0, 4, seed=3, n_seamounts=1, shelf_cols=20, land_cols=6,
+                                   source="hump")
+    want = torch.arange(nx * ny, dtype=torch.float32, device="cuda").reshape(ny, nx)
+    # the library's own page-locked block: torch's would note the session's stream and ask it after the session's end
+    p = lib.gc_host_alloc(4 * nx * ny)
+    a = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), (ny, nx))
+    a[:] = 0.0
+    torch.cuda.synchronize()
+    s = ReferenceSession(case)
+    try:
+        with torch.cuda.stream(torch.cuda.ExternalStream(s.stream())):
+            torch.cuda._sleep(100_000_000)
+            torch.from_numpy(a).copy_(want, non_blocking=True)
+        lib.cuda_setz1_(_lib.fptr(a), _i(1))
+        got = np.empty((ny, nx), np.float32)
+        lib.cuda_getz1_(_lib.fptr(got), _i(1))
+        assert np.array_equal(got, want.cpu().numpy())
+    finally:
+        s.close()
+        lib.gc_host_free(p)

@@ -49,3 +49,9 @@ def test_callers_device_memory_is_left_to_the_runtime(scenario, nx, ny):
 
 def test_copy_without_memory_for_threads(scenario):
     scenario("no-memory")
+
+
+@pytest.mark.parametrize("nx,ny", [(33, 17), (300, 300), (2401, 2001)])
+@pytest.mark.parametrize("kind", ["ordered-locked", "ordered-managed", "ordered-device"])
+def test_transfers_follow_earlier_work_on_their_stream(scenario, kind, nx, ny):
+    scenario(kind, nx, ny)
