@@ -275,7 +275,9 @@ __global__ void __launch_bounds__(32 * SWARPS) k_step_one(const __grid_constant_
 template <int N>
 struct StepGrids {
     int n, start[N + 1], tx[N];
-    GcFusedGrid g[N];
+    /* on a 16-byte boundary: at 8 bytes past one, one call on a 361 x 301 grid
+     * took 15.8 us instead of 15.0 */
+    alignas(16) GcFusedGrid g[N];
 };
 static_assert(sizeof(StepGrids<64>) <= 32000, "kernel parameters may take up to 32764 bytes");
 template <int R, int N>
