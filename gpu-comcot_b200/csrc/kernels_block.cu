@@ -48,11 +48,10 @@
  *
  * Time per step of eager launches, waves everywhere, against the two-step
  * kernel (kernels_pair.cu) on the same B200: 361 x 301 2.8 us against 8.3,
- * 961 x 801 4.6 against 9.8, 1201 x 1001 5.6 against 11.6, 2401 x 2001 19.1
- * against 22.1, eight grids of 1201 x 1001 39 against 47; of 64 such grids
- * with waves everywhere the two-step kernel is ahead, 303 against 309.  Young
- * forecasts, their waves in one corner: 2401 x 2001 11.2 against 21.4, 64 of
- * 1201 x 1001 230 against 302.
+ * 961 x 801 4.5 against 9.8, 1201 x 1001 5.4 against 11.6, 2401 x 2001 19.0
+ * against 22.1, eight grids of 1201 x 1001 39 against 47, 64 such grids 304
+ * against 303.  Young forecasts, their waves in one corner: 2401 x 2001 10.8
+ * against 21.4, 64 of 1201 x 1001 223 against 302.
  *
  * Tried and measured slower on 2401 x 2001 with 4 steps a launch: 64 columns a
  * window and two a lane (35 us a step, with twice the exchange and shuffles a
@@ -880,8 +879,8 @@ int gc_block_plan(int variant, GcFusedGrid &g, int bt) {
  * timed runs with waves everywhere on one grid of 361 x 301 to 2401 x 2001
  * cells and on 8 and 24 grids of 1201 x 1001 (within 15 % of most).  Small
  * grids want many small windows, large ones windows with little margin: per
- * step, 2.8 us (24 rows, 8 steps) against 5.3 us (64 rows) at 361 x 301, and
- * 46 us against 19.1 us at 2401 x 2001. */
+ * step, 2.8 us (24 rows, 8 steps) against 5.2 us (64 rows) at 361 x 301, and
+ * 46 us against 19.0 us at 2401 x 2001. */
 struct BlockForm {
     int variant, steps, per_sm;
     float lone, a, b;

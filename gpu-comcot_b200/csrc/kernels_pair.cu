@@ -40,8 +40,9 @@
  *
  * The register-tile kernel (kernels_block.cu) is ahead nearly everywhere.  This
  * one serves grids with fields of 4 GB and more, whose offsets do not fit that
- * kernel's 32 bits, and stays a candidate of the autotuner: 64 grids of
- * 1201 x 1001 with waves everywhere take 303 us a step here and 309 there.
+ * kernel's 32 bits, and stays a candidate of the autotuner: at 64 grids of
+ * 1201 x 1001 with waves everywhere the two are even, 303 us a step here and 304
+ * there.
  *
  * Every pipeline wait is bounded by the `wait_limit` launch parameter; a wait
  * that gives up sets g_pair_error and the warp leaves once its copies in
